@@ -132,7 +132,7 @@ size_t jvpfa_bwd_workspace_bytes(const jvpfa_bwd_args* args);
  * mask's strides are (2 * N^2 / 8 bytes per plane, N rounded up to 64). For an additive mask with contiguous,
  * 16-byte aligned rows the words mark the +-0 entries, and a tile whose other entries all carry one value
  * (0 / -inf, 0 / a large negative constant) is flagged (bit 2) with that value stored per tile: such tiles
- * are applied from the words too, all others are read element by element. The summary belongs to the
+ * are applied from the words too, all others are read element by element. Bit 3 marks a NaN. The summary belongs to the
  * mask's contents: compute it again when they change. No reference counterpart (the reference reads the mask
  * element-wise in every tile, jvp_attention.py:250-262). */
 size_t jvpfa_mask_summary_bytes(int32_t Bm, int32_t Hm, int32_t N);
@@ -141,6 +141,19 @@ int jvpfa_mask_summary(const jvpfa_mask* mask, int32_t B, int32_t H, int32_t N, 
 /* The two launches. `stream` is a cudaStream_t. */
 int jvpfa_fwd(const jvpfa_fwd_args* args, void* stream);
 int jvpfa_bwd(const jvpfa_bwd_args* args, void* stream);
+
+/* The same launches with the device status word somewhere else than at the start of the workspace: `status` is any 4 bytes
+ * the device can write to and must be zero before the first call. With mapped, pinned host memory the host can look at
+ * it without a copy or a synchronisation. */
+int jvpfa_fwd_status(const jvpfa_fwd_args* args, int32_t* status, void* stream);
+int jvpfa_bwd_status(const jvpfa_bwd_args* args, int32_t* status, void* stream);
+
+/* The reference's mask check (jvp_attention.py:2632-2656) from the summary of the mask instead of two more passes over it.
+ * `begin` launches it behind the summary pre-pass on the same stream; `end` waits for that launch alone (kernels launched
+ * in between keep running) and writes 0 (fine), 1 (a boolean mask has a (batch, head) plane with nothing kept) or 2 (an
+ * additive mask holds a NaN) to `verdict`. `end` must be called exactly once per successful `begin`. */
+int jvpfa_mask_check_begin(const jvpfa_mask* mask, int32_t B, int32_t H, int32_t N, const uint8_t* summary, void* stream, void** check);
+int jvpfa_mask_check_end(void* check, int32_t* verdict);
 
 /* Synchronises the stream, reads the status word at the start of `workspace`, clears it, and
  * returns JVPFA_OK or JVPFA_ERR_DEVICE_TIMEOUT (`detail`, if not NULL, receives the raw word:

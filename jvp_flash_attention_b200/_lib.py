@@ -34,6 +34,10 @@ EXPORTED_SYMBOLS = (
     "jvpfa_selftest_timeout",
     "jvpfa_sm_clock_probe",
     "jvpfa_bwd_noalloc",
+    "jvpfa_fwd_status",
+    "jvpfa_bwd_status",
+    "jvpfa_mask_check_begin",
+    "jvpfa_mask_check_end",
 )
 
 
@@ -129,10 +133,45 @@ def lib():
                 L.jvpfa_selftest_timeout.argtypes = [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p]
                 L.jvpfa_bwd_marked.restype = C.c_int
                 L.jvpfa_bwd_marked.argtypes = [C.POINTER(BwdArgs), C.c_void_p, C.POINTER(C.c_void_p), C.c_int32]
+                L.jvpfa_fwd_status.restype = C.c_int
+                L.jvpfa_fwd_status.argtypes = [C.POINTER(FwdArgs), C.c_void_p, C.c_void_p]
+                L.jvpfa_bwd_status.restype = C.c_int
+                L.jvpfa_bwd_status.argtypes = [C.POINTER(BwdArgs), C.c_void_p, C.c_void_p]
                 L.jvpfa_bwd_noalloc.restype = C.c_int
                 L.jvpfa_bwd_noalloc.argtypes = [C.POINTER(BwdArgs), C.c_void_p, C.c_void_p]
                 _lib = L
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (``_host.so``: argument checks, autograd nodes, launches), bound to the loaded CUDA library;
+    raises if it has not been built."""
+    global _host
+    if _host is None:
+        L = lib()
+        with _lock:
+            if _host is None:
+                try:
+                    from . import _host as module
+                except ImportError as e:
+                    raise RuntimeError("jvp_flash_attention_b200/_host.so cannot be loaded: build it with "
+                                       f"`python -m jvp_flash_attention_b200.build` ({e})") from e
+                module.bind(*(C.cast(getattr(L, n), C.c_void_p).value for n in (
+                    "jvpfa_fwd_workspace_bytes", "jvpfa_bwd_workspace_bytes", "jvpfa_mask_summary_bytes", "jvpfa_mask_summary",
+                    "jvpfa_mask_check_begin", "jvpfa_mask_check_end", "jvpfa_fwd_status", "jvpfa_bwd_status")),
+                    _workspace_addresses, check, _raise_mask)
+                _host = module
+    return _host
+
+
+def _raise_mask(verdict: int) -> None:
+    """The reference's assertions on a mask (jvp_attention.py:2632-2656)."""
+    if verdict == 1:
+        raise AssertionError("The attention mask cannot be all False for any head.")
+    raise AssertionError("The attention mask cannot contain NaNs.")
 
 
 def check(status: int) -> None:
@@ -222,11 +261,17 @@ def stream_ptr(device) -> C.c_void_p:
 # family kernels), so every stream gets its own. A buffer that is outgrown is kept alive until the process ends:
 # kernels already enqueued may still use it.
 class _Workspace:
-    def __init__(self, device, nbytes: int):
+    def __init__(self, device, nbytes: int, before: "_Workspace | None"):
         self.buf = torch.zeros(nbytes, dtype=torch.uint8, device=device)
-        self.word = self.buf[:4].view(torch.int32)                       # device status word
-        self.host = torch.zeros(1, dtype=torch.int32).pin_memory()       # its last copy on the host
-        self.retired: list = []
+        self.word = self.buf[:4].view(torch.int32)                       # status word of the self-test
+        # status word of the attention kernels: pinned host memory they write to when a wait gives up, so that a call
+        # neither copies it nor waits for it (the copy was 3 us of the stream and about as much host time a call)
+        self.host = torch.zeros(1, dtype=torch.int32).pin_memory() if before is None else before.host
+        self.retired: list = [] if before is None else before.retired + [before.buf]
+
+    @property
+    def status_ptr(self) -> int:
+        return self.host.data_ptr()
 
 
 _workspaces: dict = {}
@@ -238,36 +283,36 @@ def _ws_key(device):
 
 
 def _raise_timeout(ws: _Workspace, device) -> None:
-    """Error path: waits for the stream, reads and clears the status word, raises."""
+    """Error path: waits for the stream, reads and clears the status words, raises."""
     torch.cuda.current_stream(device).synchronize()
-    detail = int(ws.word.cpu().item())
+    detail = int(ws.word.cpu().item()) or int(ws.host[0])
     ws.word.zero_()
     ws.host.zero_()
     torch.cuda.current_stream(device).synchronize()
     raise JvpfaError(ERR_DEVICE_TIMEOUT, lib().jvpfa_error_string(ERR_DEVICE_TIMEOUT).decode() + f" (wait id {detail})")
 
 
-def workspace(device, nbytes: int) -> torch.Tensor:
-    """Workspace of the current stream of ``device`` with at least ``nbytes`` bytes. Before handing it out, looks at
-    the host copy of the status word that the previous call on this stream left (no synchronisation): a device-side
-    wait that gave up in an earlier call raises here."""
-    key = _ws_key(device)
+def _workspace_object(device, key, nbytes: int) -> _Workspace:
+    """Before handing the workspace of ``key`` out, looks at its status word on the host (no synchronisation): a
+    device-side wait that gave up in an earlier call raises here."""
     ws = _workspaces.get(key)
     if ws is not None and int(ws.host[0]) != 0:
         _raise_timeout(ws, device)
     if ws is None or ws.buf.numel() < nbytes:
-        new = _Workspace(device, max(nbytes, 1 << 20))
-        if ws is not None:
-            new.retired = ws.retired + [ws.buf]
-        _workspaces[key] = ws = new
-    return ws.buf
+        _workspaces[key] = ws = _Workspace(device, max(nbytes, 1 << 20), ws)
+    return ws
 
 
-def post_launch(device) -> None:
-    """Enqueues a copy of the status word to pinned host memory behind the kernels just launched."""
-    ws = _workspaces.get(_ws_key(device))
-    if ws is not None:
-        ws.host.copy_(ws.word, non_blocking=True)
+def workspace(device, nbytes: int) -> torch.Tensor:
+    """Workspace of the current stream of ``device`` with at least ``nbytes`` bytes."""
+    return _workspace_object(device, _ws_key(device), nbytes).buf
+
+
+def _workspace_addresses(index: int, stream: int, nbytes: int):
+    """What the native host path asks for when it does not know a large enough workspace of a stream (which is the current
+    one) or finds its status word set: (address, bytes, address of the status word)."""
+    ws = _workspace_object(torch.device("cuda", index), (index, stream), nbytes)
+    return ws.buf.data_ptr(), ws.buf.numel(), ws.status_ptr
 
 
 def read_status(device=None) -> None:
@@ -280,9 +325,12 @@ def read_status(device=None) -> None:
             continue
         detail = C.c_int32(0)
         rc = lib().jvpfa_read_status(C.c_void_p(ws.buf.data_ptr()), stream_ptr(device), C.byref(detail))
+        code = detail.value or int(ws.host[0])
         ws.host.zero_()
+        if rc == OK and code != 0:
+            rc = ERR_DEVICE_TIMEOUT
         if rc != OK:
-            raise JvpfaError(rc, lib().jvpfa_error_string(rc).decode() + f" (wait id {detail.value})")
+            raise JvpfaError(rc, lib().jvpfa_error_string(rc).decode() + f" (wait id {code})")
 
 
 def sm_clock_probe(stream: "torch.cuda.Stream", duration_us: int) -> torch.Tensor:
@@ -301,7 +349,8 @@ def selftest_timeout(device, budget_us: int = 2000) -> torch.Tensor:
     out = torch.full((4,), -1, dtype=torch.int32, device=device)
     check(lib().jvpfa_selftest_timeout(C.c_void_p(ws.data_ptr()), int(budget_us), C.c_void_p(out.data_ptr()),
                                        stream_ptr(device)))
-    post_launch(device)
+    w = _workspaces[_ws_key(device)]
+    w.host.copy_(w.word, non_blocking=True)      # the self-test writes to the workspace: where the next call looks is on the host
     return out
 
 
@@ -347,10 +396,9 @@ def fwd(q, k, v, tq, tk, tv, mask_c: Mask, summary, causal: bool, sm_scale: floa
     a.o, a.to = o.data_ptr(), (to.data_ptr() if dual else None)
     a.lse2, a.mu = lse2.data_ptr(), mu.data_ptr()
     need = lib().jvpfa_fwd_workspace_bytes(C.byref(a))
-    ws = workspace(q.device, need)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-    check(lib().jvpfa_fwd(C.byref(a), stream_ptr(q.device)))
-    post_launch(q.device)
+    ws = _workspace_object(q.device, _ws_key(q.device), need)
+    a.workspace, a.workspace_bytes = ws.buf.data_ptr(), ws.buf.numel()
+    check(lib().jvpfa_fwd_status(C.byref(a), C.c_void_p(ws.status_ptr), stream_ptr(q.device)))
     return o, to, lse2, mu
 
 
@@ -384,12 +432,11 @@ def bwd(q, k, v, tq, tk, tv, o, to, lse2, mu, go, gto, mask_c: Mask, summary, ca
     else:
         a.tq = a.tk = a.tv = a.to = a.gto = a.dtq = a.dtk = a.dtv = None
     need = lib().jvpfa_bwd_workspace_bytes(C.byref(a))
-    ws = workspace(q.device, need)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    ws = _workspace_object(q.device, _ws_key(q.device), need)
+    a.workspace, a.workspace_bytes = ws.buf.data_ptr(), ws.buf.numel()
     if marks is None:
-        check(lib().jvpfa_bwd(C.byref(a), stream_ptr(q.device)))
+        check(lib().jvpfa_bwd_status(C.byref(a), C.c_void_p(ws.status_ptr), stream_ptr(q.device)))
     else:
         handles = (C.c_void_p * 5)(*[C.c_void_p(e.cuda_event) for e in marks])
         check(lib().jvpfa_bwd_marked(C.byref(a), stream_ptr(q.device), handles, 5))
-    post_launch(q.device)
     return tuple(outs)

@@ -1,4 +1,4 @@
-"""Builds libjvpfa.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Builds libjvpfa.so (the C-ABI CUDA library, nvcc for sm_100a) and _host.so (the native host path, g++) in-tree.
 
 Usage: ``python -m jvp_flash_attention_b200.build [--force] [--verbose]``. Each ``csrc/*.cu`` is
 compiled to an object (in parallel) and linked into ``jvp_flash_attention_b200/libjvpfa.so``.
@@ -18,6 +18,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "csrc" / "build"
 LIB = PKG / "libjvpfa.so"
+HOST_SRC = CSRC / "host_torch.cpp"      # the native host path: plain C++ against torch, no CUDA code
+HOST_LIB = PKG / "_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -37,6 +39,20 @@ def _nvcc() -> str:
 def _newest_header_mtime() -> float:
     hdrs = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + list((PKG.parent / "include").glob("*.h"))
     return max(h.stat().st_mtime for h in hdrs)
+
+
+def _build_host() -> None:
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import CUDA_HOME, include_paths, library_paths
+    inc = [f"-I{p}" for p in (*include_paths(), sysconfig.get_paths()["include"], f"{CUDA_HOME or '/usr/local/cuda'}/include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *inc, str(HOST_SRC), "-o", str(HOST_LIB),
+           *(f"-L{p}" for p in library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError(f"g++ failed on {HOST_SRC.name}")
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -70,6 +86,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    if force or not HOST_LIB.exists() or HOST_LIB.stat().st_mtime < max(HOST_SRC.stat().st_mtime, hdr_m):
+        _build_host()
     return LIB
 
 

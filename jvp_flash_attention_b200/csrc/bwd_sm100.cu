@@ -967,41 +967,52 @@ __global__ void bwd_preprocess_f32_kernel(const float* __restrict__ o, const flo
   }
 }
 
+// The tensor maps of a backward call, one with the row-side and one with the column-side box per operand: every operand
+// is row-side in one family and column-side in another, so they are encoded once for all launches of the call.
+enum { OP_Q = 0, OP_K, OP_V, OP_GO, OP_TQ, OP_TK, OP_TV, OP_GTO, N_OPS };
+struct BwdMaps {
+  CUtensorMap row[N_OPS], col[N_OPS];
+  bool encode(const jvpfa_bwd_args& a) {
+    const void* const ptr[N_OPS] = {a.q, a.k, a.v, a.go, a.tq, a.tk, a.tv, a.gto};
+    const jvpfa_strides* const st[N_OPS] = {&a.q_strides, &a.k_strides, &a.v_strides, &a.go_strides,
+                                            &a.tq_strides, &a.tk_strides, &a.tv_strides, &a.gto_strides};
+    const bool dual = a.tq != nullptr;
+    for (int i = 0; i < N_OPS; ++i) {
+      if (!dual && i >= OP_TQ) {   // tangent operands of a primal-only call: aliases, never used
+        row[i] = row[i - OP_TQ];
+        col[i] = col[i - OP_TQ];
+        continue;
+      }
+      const TensorView v = make_view(ptr[i], *st[i], a.H, a.N, a.D);
+      if (!make_tile_map(&row[i], v, a.B, a.H, a.N, a.D, 128, a.dtype) || !make_tile_map(&col[i], v, a.B, a.H, a.N, a.D, 64, a.dtype))
+        return false;
+    }
+    return true;
+  }
+};
+
 // `a` holds the operands the tensor maps are built on: in the split-fp32 mode (SPLIT) the bf16 hi/lo tensors of the
 // pre-pass with 128 columns, and `real_D` is the head dimension of the outputs.
 template <int D, int FAM, bool BF16, bool PAD, bool DUAL, bool SPLIT = false, bool DROP = false>
-int launch_family(const jvpfa_bwd_args& a, const float4* stats, cudaStream_t stream, int real_D = 0) {
+int launch_family(const jvpfa_bwd_args& a, const BwdMaps& m, const float4* stats, int* status, cudaStream_t stream, int real_D = 0) {
   using C = BwdCfg<D, FAM, SPLIT>;
-  const TensorView vq = make_view(a.q, a.q_strides, a.H, a.N, a.D), vk = make_view(a.k, a.k_strides, a.H, a.N, a.D),
-                   vv = make_view(a.v, a.v_strides, a.H, a.N, a.D), vtq = make_view(a.tq, a.tq_strides, a.H, a.N, a.D),
-                   vtk = make_view(a.tk, a.tk_strides, a.H, a.N, a.D), vtv = make_view(a.tv, a.tv_strides, a.H, a.N, a.D),
-                   vgo = make_view(a.go, a.go_strides, a.H, a.N, a.D), vgto = make_view(a.gto, a.gto_strides, a.H, a.N, a.D);
-  TensorView rsrc[4];
-  TensorView csrc[4];
+  static_assert(C::BR == 128 && C::BC == 64, "the boxes of BwdMaps");
+  // rows and first / second column pair of the family: query side {q, tq, go, gto} or key side {k, tk, v, tv} (family V
+  // reads k, tk only)
+  const bool rows_q = FAM == FAM_Q;
+  const CUtensorMap* const rm[4] = {&m.row[rows_q ? OP_Q : OP_K], &m.row[rows_q ? OP_TQ : OP_TK], &m.row[rows_q ? OP_GO : OP_V],
+                                    &m.row[rows_q ? OP_GTO : OP_TV]};
+  const CUtensorMap* const cm[4] = {&m.col[rows_q ? OP_K : OP_Q], &m.col[rows_q ? OP_TK : OP_TQ], &m.col[rows_q ? OP_V : OP_GO],
+                                    &m.col[rows_q ? OP_TV : OP_GTO]};
   void *out0, *out1, *out2 = nullptr, *out3 = nullptr;
-  float out_scale;
+  float out_scale = a.sm_scale;
   if (FAM == FAM_Q) {
-    rsrc[0] = vq; rsrc[1] = vtq; rsrc[2] = vgo; rsrc[3] = vgto;
-    csrc[0] = vk; csrc[1] = vtk; csrc[2] = vv; csrc[3] = vtv;
-    out0 = a.dq; out1 = a.dtq; out_scale = a.sm_scale;
+    out0 = a.dq; out1 = a.dtq;
   } else if (FAM == FAM_K || FAM == FAM_KV) {
-    rsrc[0] = vk; rsrc[1] = vtk; rsrc[2] = vv; rsrc[3] = vtv;
-    csrc[0] = vq; csrc[1] = vtq; csrc[2] = vgo; csrc[3] = vgto;
-    out0 = a.dk; out1 = a.dtk; out_scale = a.sm_scale;
+    out0 = a.dk; out1 = a.dtk;
     if (FAM == FAM_KV) { out2 = a.dv; out3 = a.dtv; }
   } else {
-    rsrc[0] = vk; rsrc[1] = vtk; rsrc[2] = vk; rsrc[3] = vtk;
-    csrc[0] = vq; csrc[1] = vtq; csrc[2] = vgo; csrc[3] = vgto;
     out0 = a.dv; out1 = a.dtv; out_scale = 1.0f;
-  }
-  if (!DUAL) {  // tensors that do not exist in the primal-only call: alias the maps to existing ones, they are never used
-    rsrc[1] = rsrc[0]; rsrc[3] = rsrc[2];
-    csrc[1] = csrc[0]; csrc[3] = csrc[2];
-  }
-  CUtensorMap rm[4], cm[4];
-  for (int i = 0; i < 4; ++i) {
-    if (!make_tile_map(&rm[i], rsrc[i], a.B, a.H, a.N, a.D, C::BR, a.dtype)) return JVPFA_ERR_LAUNCH;
-    if (!make_tile_map(&cm[i], csrc[i], a.B, a.H, a.N, a.D, C::BC, a.dtype)) return JVPFA_ERR_LAUNCH;
   }
   BwdKParams p{};
   p.H = a.H; p.N = a.N; p.D = SPLIT ? real_D : a.D; p.causal = a.causal;
@@ -1011,23 +1022,23 @@ int launch_family(const jvpfa_bwd_args& a, const float4* stats, cudaStream_t str
   p.mv = make_mask_view(a.mask, a.mask_summary, a.B, a.H, a.N);
   p.stats = stats;
   p.out0 = out0; p.out1 = out1; p.out2 = out2; p.out3 = out3;
-  p.status = static_cast<int*>(a.workspace);
+  p.status = status;
   p.budget_ns = wait_budget_ns();
   p.drop = make_dropout_params(a.dropout_p, a.dropout_seed);
   auto kern = bwd_sm100_kernel<D, FAM, BF16, PAD, DUAL, SPLIT, DROP>;
   const size_t smem = C::smem_bytes();
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-    return JVPFA_ERR_LAUNCH;
+  static SmemOptIn opt_in;
+  if (!opt_in.set(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_LAUNCH;
   p.n_rt = (a.N + C::BR - 1) / C::BR;
   p.n_units = a.B * a.H;
   p.unit_group = unit_group_size(p.n_units);
   dim3 grid(static_cast<unsigned>(p.n_rt) * static_cast<unsigned>(p.n_units));
-  kern<<<grid, 352, smem, stream>>>(rm[0], rm[1], rm[2], rm[3], cm[0], cm[1], cm[2], cm[3], p);
+  kern<<<grid, 352, smem, stream>>>(*rm[0], *rm[1], *rm[2], *rm[3], *cm[0], *cm[1], *cm[2], *cm[3], p);
   return cudaGetLastError() == cudaSuccess ? JVPFA_OK : JVPFA_ERR_LAUNCH;
 }
 
 template <int D, bool BF16>
-int launch_all(const jvpfa_bwd_args& a, cudaStream_t stream, const LaunchMarks& marks) {
+int launch_all(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks) {
   const int64_t rows = static_cast<int64_t>(a.B) * a.H * a.N;
   float4* stats = reinterpret_cast<float4*>(static_cast<uint8_t*>(a.workspace) + kStatusBytes);
   const int warps_per_block = 8;   // two rows per warp
@@ -1038,20 +1049,22 @@ int launch_all(const jvpfa_bwd_args& a, cudaStream_t stream, const LaunchMarks& 
       static_cast<const uint16_t*>(a.o), static_cast<const uint16_t*>(a.to), static_cast<const uint16_t*>(a.go),
       static_cast<const uint16_t*>(a.gto), a.lse2, a.mu, stats, rows, a.D, gl);
   if (cudaGetLastError() != cudaSuccess) return JVPFA_ERR_LAUNCH;
+  BwdMaps maps;
+  if (!maps.encode(a)) return JVPFA_ERR_LAUNCH;
   auto three = [&](auto pad, auto dual, auto drop) {
     constexpr bool P = decltype(pad)::value, DU = decltype(dual)::value, DR = decltype(drop)::value;
     marks.mark(1);
-    int rc = launch_family<D, FAM_Q, BF16, P, DU, false, DR>(a, stats, stream);
+    int rc = launch_family<D, FAM_Q, BF16, P, DU, false, DR>(a, maps, stats, status, stream);
     if (rc != JVPFA_OK) return rc;
     marks.mark(2);
     if constexpr (D == 64) {   // the key-side gradients in one pass
-      rc = launch_family<D, FAM_KV, BF16, P, DU, false, DR>(a, stats, stream);
+      rc = launch_family<D, FAM_KV, BF16, P, DU, false, DR>(a, maps, stats, status, stream);
       marks.mark(3);
     } else {
-      rc = launch_family<D, FAM_K, BF16, P, DU, false, DR>(a, stats, stream);
+      rc = launch_family<D, FAM_K, BF16, P, DU, false, DR>(a, maps, stats, status, stream);
       if (rc != JVPFA_OK) return rc;
       marks.mark(3);
-      rc = launch_family<D, FAM_V, BF16, P, DU, false, DR>(a, stats, stream);
+      rc = launch_family<D, FAM_V, BF16, P, DU, false, DR>(a, maps, stats, status, stream);
     }
     marks.mark(4);
     return rc;
@@ -1069,7 +1082,7 @@ int launch_all(const jvpfa_bwd_args& a, cudaStream_t stream, const LaunchMarks& 
 // workspace, then the three family kernels in their split mode on the split tensors. Workspace: status block, statistics,
 // split tensors.
 template <bool DUAL, bool DROP>
-int launch_split(const jvpfa_bwd_args& a, cudaStream_t stream, const LaunchMarks& marks) {
+int launch_split(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks) {
   const int64_t rows = static_cast<int64_t>(a.B) * a.H * a.N;
   uint8_t* ws = static_cast<uint8_t*>(a.workspace);
   float4* stats = reinterpret_cast<float4*>(ws + kStatusBytes);
@@ -1099,14 +1112,16 @@ int launch_split(const jvpfa_bwd_args& a, cudaStream_t stream, const LaunchMarks
   m.q_strides = m.k_strides = m.v_strides = m.tq_strides = m.tk_strides = m.tv_strides = m.go_strides = m.gto_strides = none;
   m.q = dst[0]; m.k = dst[1]; m.v = dst[2]; m.go = dst[3];
   if (DUAL) { m.tq = dst[4]; m.tk = dst[5]; m.tv = dst[6]; m.gto = dst[7]; }
+  BwdMaps maps;
+  if (!maps.encode(m)) return JVPFA_ERR_LAUNCH;
   marks.mark(1);
-  rc = launch_family<128, FAM_Q, true, false, DUAL, true, DROP>(m, stats, stream, a.D);
+  rc = launch_family<128, FAM_Q, true, false, DUAL, true, DROP>(m, maps, stats, status, stream, a.D);
   if (rc != JVPFA_OK) return rc;
   marks.mark(2);
-  rc = launch_family<128, FAM_K, true, false, DUAL, true, DROP>(m, stats, stream, a.D);
+  rc = launch_family<128, FAM_K, true, false, DUAL, true, DROP>(m, maps, stats, status, stream, a.D);
   if (rc != JVPFA_OK) return rc;
   marks.mark(3);
-  rc = launch_family<128, FAM_V, true, false, DUAL, true, DROP>(m, stats, stream, a.D);
+  rc = launch_family<128, FAM_V, true, false, DUAL, true, DROP>(m, maps, stats, status, stream, a.D);
   marks.mark(4);
   return rc;
 }
@@ -1118,20 +1133,20 @@ size_t bwd_sm100_split_workspace_bytes(const jvpfa_bwd_args& a) {
   return kStatusBytes + align_up(rows * sizeof(float4), 256) + (a.tq != nullptr ? 8 : 4) * rows * kSplitRowBytes;
 }
 
-int launch_bwd_sm100_split(const jvpfa_bwd_args& a, cudaStream_t stream, const LaunchMarks& marks) {
+int launch_bwd_sm100_split(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks) {
   if (a.dropout_p > 0.f)
-    return a.tq != nullptr ? launch_split<true, true>(a, stream, marks) : launch_split<false, true>(a, stream, marks);
-  return a.tq != nullptr ? launch_split<true, false>(a, stream, marks) : launch_split<false, false>(a, stream, marks);
+    return a.tq != nullptr ? launch_split<true, true>(a, status, stream, marks) : launch_split<false, true>(a, status, stream, marks);
+  return a.tq != nullptr ? launch_split<true, false>(a, status, stream, marks) : launch_split<false, false>(a, status, stream, marks);
 }
 
 size_t bwd_sm100_workspace_bytes(const jvpfa_bwd_args& a) {
   return kStatusBytes + static_cast<size_t>(a.B) * a.H * a.N * sizeof(float4);
 }
 
-int launch_bwd_sm100(const jvpfa_bwd_args& a, cudaStream_t stream, const LaunchMarks& marks) {
+int launch_bwd_sm100(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks) {
   const bool bf = a.dtype == JVPFA_BF16;
-  if (sm100_padded_dim(a.D) == 64) return bf ? launch_all<64, true>(a, stream, marks) : launch_all<64, false>(a, stream, marks);
-  return bf ? launch_all<128, true>(a, stream, marks) : launch_all<128, false>(a, stream, marks);
+  if (sm100_padded_dim(a.D) == 64) return bf ? launch_all<64, true>(a, status, stream, marks) : launch_all<64, false>(a, status, stream, marks);
+  return bf ? launch_all<128, true>(a, status, stream, marks) : launch_all<128, false>(a, status, stream, marks);
 }
 
 }  // namespace jvpfa

@@ -625,7 +625,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 }
 
 template <int D, bool DUAL, bool BF16, bool PAD, bool DROP = false>
-int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
+int launch_one(const jvpfa_fwd_args& a, int* status, cudaStream_t stream) {
   using C = FwdCfg<D>;
   CUtensorMap mQ, mTQ, mK, mTK, mV, mTV;
   auto tile = [&](CUtensorMap* m, const void* ptr, const jvpfa_strides& st, int box_rows) {
@@ -649,13 +649,13 @@ int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
   p.thresh = BF16 ? 8.0f : 6.0f;
   p.mv = make_mask_view(a.mask, a.mask_summary, a.B, a.H, a.N);
   p.o = a.o; p.to = a.to; p.lse2 = a.lse2; p.mu = a.mu;
-  p.status = static_cast<int*>(a.workspace);
+  p.status = status;
   p.budget_ns = wait_budget_ns();
   p.drop = make_dropout_params(a.dropout_p, a.dropout_seed);
   auto kern = fwd_sm100_kernel<D, DUAL, BF16, PAD, false, DROP>;
   const size_t smem = C::smem_bytes();
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-    return JVPFA_ERR_LAUNCH;
+  static SmemOptIn opt_in;
+  if (!opt_in.set(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_LAUNCH;
   p.n_qt = (a.N + C::BM - 1) / C::BM;
   p.n_units = a.B * a.H;
   p.unit_group = unit_group_size(p.n_units);
@@ -666,7 +666,7 @@ int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
 
 // fp32 inputs: split pre-pass into the workspace, then the 128-column kernel in its split mode on the split tensors.
 template <bool DUAL, bool DROP>
-int launch_split(const jvpfa_fwd_args& a, cudaStream_t stream) {
+int launch_split(const jvpfa_fwd_args& a, int* status, cudaStream_t stream) {
   using C = FwdCfg<128, true>;
   const int64_t rows = static_cast<int64_t>(a.B) * a.H * a.N;
   const int n_t = DUAL ? 6 : 3;
@@ -701,13 +701,13 @@ int launch_split(const jvpfa_fwd_args& a, cudaStream_t stream) {
   p.thresh = 8.0f;
   p.mv = make_mask_view(a.mask, a.mask_summary, a.B, a.H, a.N);
   p.o = a.o; p.to = a.to; p.lse2 = a.lse2; p.mu = a.mu;
-  p.status = static_cast<int*>(a.workspace);
+  p.status = status;
   p.budget_ns = wait_budget_ns();
   p.drop = make_dropout_params(a.dropout_p, a.dropout_seed);
   auto kern = fwd_sm100_kernel<128, DUAL, true, false, true, DROP>;
   const size_t smem = C::smem_bytes();
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-    return JVPFA_ERR_LAUNCH;
+  static SmemOptIn opt_in;
+  if (!opt_in.set(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_LAUNCH;
   p.n_qt = (a.N + C::BM - 1) / C::BM;
   p.n_units = a.B * a.H;
   p.unit_group = unit_group_size(p.n_units);
@@ -727,9 +727,9 @@ size_t fwd_sm100_split_workspace_bytes(const jvpfa_fwd_args& a) {
   return kStatusBytes + (a.tq != nullptr ? 6 : 3) * rows * kSplitRowBytes;
 }
 
-int launch_fwd_sm100_split(const jvpfa_fwd_args& a, cudaStream_t stream) {
-  if (a.dropout_p > 0.f) return a.tq != nullptr ? launch_split<true, true>(a, stream) : launch_split<false, true>(a, stream);
-  return a.tq != nullptr ? launch_split<true, false>(a, stream) : launch_split<false, false>(a, stream);
+int launch_fwd_sm100_split(const jvpfa_fwd_args& a, int* status, cudaStream_t stream) {
+  if (a.dropout_p > 0.f) return a.tq != nullptr ? launch_split<true, true>(a, status, stream) : launch_split<false, true>(a, status, stream);
+  return a.tq != nullptr ? launch_split<true, false>(a, status, stream) : launch_split<false, false>(a, status, stream);
 }
 
 bool sm100_path_supported(int dtype, int D, int N) {
@@ -739,21 +739,21 @@ bool sm100_path_supported(int dtype, int D, int N) {
 
 namespace {
 template <int D, bool PAD>
-int launch_by_mode(const jvpfa_fwd_args& a, cudaStream_t stream) {
+int launch_by_mode(const jvpfa_fwd_args& a, int* status, cudaStream_t stream) {
   const bool dual = a.tq != nullptr;
   const bool bf = a.dtype == JVPFA_BF16;
   if (a.dropout_p > 0.f) {
-    if (dual) return bf ? launch_one<D, true, true, PAD, true>(a, stream) : launch_one<D, true, false, PAD, true>(a, stream);
-    return bf ? launch_one<D, false, true, PAD, true>(a, stream) : launch_one<D, false, false, PAD, true>(a, stream);
+    if (dual) return bf ? launch_one<D, true, true, PAD, true>(a, status, stream) : launch_one<D, true, false, PAD, true>(a, status, stream);
+    return bf ? launch_one<D, false, true, PAD, true>(a, status, stream) : launch_one<D, false, false, PAD, true>(a, status, stream);
   }
-  if (dual) return bf ? launch_one<D, true, true, PAD>(a, stream) : launch_one<D, true, false, PAD>(a, stream);
-  return bf ? launch_one<D, false, true, PAD>(a, stream) : launch_one<D, false, false, PAD>(a, stream);
+  if (dual) return bf ? launch_one<D, true, true, PAD>(a, status, stream) : launch_one<D, true, false, PAD>(a, status, stream);
+  return bf ? launch_one<D, false, true, PAD>(a, status, stream) : launch_one<D, false, false, PAD>(a, status, stream);
 }
 }  // namespace
 
-int launch_fwd_sm100(const jvpfa_fwd_args& a, cudaStream_t stream) {
-  if (sm100_padded_dim(a.D) == 64) return a.D == 64 ? launch_by_mode<64, false>(a, stream) : launch_by_mode<64, true>(a, stream);
-  return a.D == 128 ? launch_by_mode<128, false>(a, stream) : launch_by_mode<128, true>(a, stream);
+int launch_fwd_sm100(const jvpfa_fwd_args& a, int* status, cudaStream_t stream) {
+  if (sm100_padded_dim(a.D) == 64) return a.D == 64 ? launch_by_mode<64, false>(a, status, stream) : launch_by_mode<64, true>(a, status, stream);
+  return a.D == 128 ? launch_by_mode<128, false>(a, status, stream) : launch_by_mode<128, true>(a, status, stream);
 }
 
 }  // namespace jvpfa

@@ -1,6 +1,7 @@
 // Host-side helpers shared by the launchers: TMA tensor-map encoding through the driver entry
 // point (the library does not link libcuda), the device status word, small utilities.
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <cuda.h>
@@ -58,6 +59,24 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // Workspace layout shared by forward and backward: [0,256) status word + padding, then per-call scratch.
 constexpr size_t kStatusBytes = 256;
 
+// The opt-in to more than 48 KB of dynamic shared memory, once per kernel and device (one static object beside each
+// launch) instead of before every launch.
+class SmemOptIn {
+ public:
+  bool set(const void* kernel, size_t bytes) {
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (done_.load(std::memory_order_acquire) & bit) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) != cudaSuccess) return false;
+    done_.fetch_or(bit, std::memory_order_release);
+    return true;
+  }
+
+ private:
+  std::atomic<uint64_t> done_{0};
+};
+
 // Optional caller-owned events of jvpfa_bwd_marked: mark(i) records event i on the stream when events were given.
 struct LaunchMarks {
   void* const* events = nullptr;
@@ -75,11 +94,11 @@ int launch_split_fp32(const TensorView* src, uint16_t* const* dst, int n_tensors
 bool sm100_split_path_supported(int dtype, int D, int N);
 size_t fwd_sm100_split_workspace_bytes(const jvpfa_fwd_args& a);
 size_t bwd_sm100_split_workspace_bytes(const jvpfa_bwd_args& a);
-int launch_fwd_sm100_split(const jvpfa_fwd_args& a, cudaStream_t stream);
-int launch_bwd_sm100_split(const jvpfa_bwd_args& a, cudaStream_t stream, const LaunchMarks& marks);
+int launch_fwd_sm100_split(const jvpfa_fwd_args& a, int* status, cudaStream_t stream);
+int launch_bwd_sm100_split(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks);
 
-int launch_fwd_sm100(const jvpfa_fwd_args& a, cudaStream_t stream);
-int launch_bwd_sm100(const jvpfa_bwd_args& a, cudaStream_t stream, const LaunchMarks& marks);
+int launch_fwd_sm100(const jvpfa_fwd_args& a, int* status, cudaStream_t stream);
+int launch_bwd_sm100(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks);
 size_t bwd_sm100_workspace_bytes(const jvpfa_bwd_args& a);
 bool sm100_path_supported(int dtype, int D, int N);
 inline int sm100_padded_dim(int D) { return D <= 64 ? 64 : 128; }

@@ -3,6 +3,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <vector>
 #include "host_common.h"
 #include "mask_common.cuh"
 #include "sm100_prims.cuh"
@@ -129,7 +130,7 @@ mask_summary_kernel(MaskView mv, int N, uint8_t* flags, uint32_t* rowbits, uint6
     if (t < cc && k0 + t < mv.n_pad) {   // (whole warps: cc and n_pad are multiples of 32)
       const int k = k0 + t;
       uint64_t word = 0;
-      bool any_masked = false;
+      bool any_masked = false, any_nan = false;
       uint32_t mine0 = 0, mine1 = 0;   // ballots of rows lane and lane + 32
 #pragma unroll 8
       for (int r = 0; r < 64; ++r) {
@@ -142,6 +143,7 @@ mask_summary_kernel(MaskView mv, int N, uint8_t* flags, uint32_t* rowbits, uint6
           const float m = mask_elem_as_float(tile, r * cc + t, mv.dtype);
           kept = m != -INFINITY;
           masked = m != 0.f;
+          any_nan |= in && m != m;
         }
         kept = kept && in;
         any_masked |= masked && in;
@@ -156,7 +158,8 @@ mask_summary_kernel(MaskView mv, int N, uint8_t* flags, uint32_t* rowbits, uint6
         rb[2 * lane] = mine0;
         rb[2 * (lane + 32)] = mine1;
       }
-      const uint32_t fl = (__any_sync(0xFFFFFFFFu, word != 0) ? kTileAnyKept : 0u) | (__any_sync(0xFFFFFFFFu, any_masked) ? kTileAnyMasked : 0u);
+      const uint32_t fl = (__any_sync(0xFFFFFFFFu, word != 0) ? kTileAnyKept : 0u) | (__any_sync(0xFFFFFFFFu, any_masked) ? kTileAnyMasked : 0u) |
+                          (__any_sync(0xFFFFFFFFu, any_nan) ? kTileAnyNaN : 0u);
       if (lane == 0 && fl) atomicOr(&tflags[kt], fl);
     }
   }
@@ -257,8 +260,9 @@ mask_summary_additive_kernel(MaskView mv, int N, uint8_t* flags, uint32_t* rowbi
   constexpr int WORDS = 32 * ES / 4;   // 32-bit words of a query's 32 entries
   const uint32_t ninf = ES == 4 ? 0xFF800000u : (mv.dtype == JVPFA_BF16 ? 0xFF80u : 0xFC00u);
   const uint32_t absmask = ES == 4 ? 0x7FFFFFFFu : 0x7FFFu;
+  const uint32_t inf = ninf & absmask;
   for (int kt = blockIdx.z + gridDim.z * warp; kt < mv.n64; kt += gridDim.z * 8) {
-    bool kept_any = false, masked_any = false, has = false, multi = false;
+    bool kept_any = false, masked_any = false, has = false, multi = false, nan = false;
     uint32_t val = 0;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
@@ -297,6 +301,7 @@ mask_summary_additive_kernel(MaskView mv, int N, uint8_t* flags, uint32_t* rowbi
           const bool zero = (e & absmask) == 0u;
           bits |= (in && zero ? 1u : 0u) << i;
           kept_any |= in && e != ninf;
+          nan |= in && (e & absmask) > inf;
           const bool nz = in && !zero;
           masked_any |= nz;
           multi |= nz && has && e != val;
@@ -315,13 +320,14 @@ mask_summary_additive_kernel(MaskView mv, int N, uint8_t* flags, uint32_t* rowbi
     const bool any_kept = __any_sync(0xFFFFFFFFu, kept_any);
     const bool any_masked = __any_sync(0xFFFFFFFFu, masked_any);
     const bool any_multi = __any_sync(0xFFFFFFFFu, multi);
+    const bool any_nan = __any_sync(0xFFFFFFFFu, nan);
     const uint32_t has_b = __ballot_sync(0xFFFFFFFFu, has);
     const uint32_t v0 = __shfl_sync(0xFFFFFFFFu, val, has_b ? __ffs(has_b) - 1 : 0);
     const bool same = __all_sync(0xFFFFFFFFu, !has || val == v0);
     if (lane == 0) {
       const bool two = !any_multi && same;
       const int64_t t = (static_cast<int64_t>(plane) * mv.n64 + band) * mv.n64 + kt;
-      flags[t] = static_cast<uint8_t>((any_kept ? kTileAnyKept : 0) | (any_masked ? kTileAnyMasked : 0) | (two ? kTileTwoValued : 0));
+      flags[t] = static_cast<uint8_t>((any_kept ? kTileAnyKept : 0) | (any_masked ? kTileAnyMasked : 0) | (two ? kTileTwoValued : 0) | (any_nan ? kTileAnyNaN : 0));
       float c = 0.f;
       if (has_b) {
         if (ES == 4) c = __uint_as_float(v0);
@@ -358,6 +364,70 @@ __global__ void selftest_timeout_kernel(int* status, uint64_t budget_ns, int* ou
     out[2] = static_cast<int>((t1 - t0) / 1000);
     out[3] = static_cast<int>((t2 - t1) / 1000);
   }
+}
+
+// Verdict on a mask from its summary, one block per plane: 1 = a boolean mask has a plane with nothing kept, 2 = an additive
+// mask holds a NaN. `verdict` is host memory; it stays untouched when the mask is fine.
+__global__ void __launch_bounds__(256) mask_check_kernel(const uint8_t* flags, int tiles, int kind, int* verdict) {
+  const uint8_t* f = flags + static_cast<size_t>(blockIdx.x) * tiles;
+  bool kept = false, nan = false;
+  for (int i = threadIdx.x; i < tiles; i += blockDim.x) {
+    kept |= (f[i] & kTileAnyKept) != 0;
+    nan |= (f[i] & kTileAnyNaN) != 0;
+  }
+  const bool any_kept = __syncthreads_or(kept), any_nan = __syncthreads_or(nan);
+  if (threadIdx.x == 0) {
+    if (kind == JVPFA_MASK_BOOL && !any_kept) *verdict = 1;
+    if (kind == JVPFA_MASK_ADDITIVE && any_nan) *verdict = 2;
+  }
+}
+
+// A host word the check kernel writes to and the event that says it has run. Kept for the next call; at most as many as
+// there have been checks in flight at once, and no more than kMaxMaskChecks of them are kept.
+struct MaskCheck {
+  cudaEvent_t done = nullptr;
+  int* verdict = nullptr;   // pinned host memory
+  int device = -1;
+};
+constexpr size_t kMaxMaskChecks = 64;
+std::mutex g_mask_check_mutex;
+std::vector<MaskCheck*> g_mask_checks;
+
+void free_mask_check(MaskCheck* c) {
+  if (c->done != nullptr) cudaEventDestroy(c->done);
+  if (c->verdict != nullptr) cudaFreeHost(c->verdict);
+  delete c;
+}
+MaskCheck* take_mask_check() {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_mask_check_mutex);
+    for (size_t i = 0; i < g_mask_checks.size(); ++i)
+      if (g_mask_checks[i]->device == dev) {
+        MaskCheck* c = g_mask_checks[i];
+        g_mask_checks.erase(g_mask_checks.begin() + i);
+        return c;
+      }
+  }
+  MaskCheck* c = new MaskCheck;
+  c->device = dev;
+  if (cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming) != cudaSuccess ||
+      cudaHostAlloc(reinterpret_cast<void**>(&c->verdict), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+    free_mask_check(c);
+    return nullptr;
+  }
+  return c;
+}
+void give_back_mask_check(MaskCheck* c) {
+  {
+    std::lock_guard<std::mutex> lock(g_mask_check_mutex);
+    if (g_mask_checks.size() < kMaxMaskChecks) {
+      g_mask_checks.push_back(c);
+      return;
+    }
+  }
+  free_mask_check(c);
 }
 
 // Average SM clock over a stretch of time: one thread reads the SM's cycle counter and the global nanosecond timer,
@@ -486,7 +556,42 @@ int jvpfa_mask_summary(const jvpfa_mask* mask, int32_t B, int32_t H, int32_t N, 
   return cudaGetLastError() == cudaSuccess ? JVPFA_OK : JVPFA_ERR_LAUNCH;
 }
 
+int jvpfa_mask_check_begin(const jvpfa_mask* mask, int32_t B, int32_t H, int32_t N, const uint8_t* summary, void* stream, void** check) {
+  if (mask == nullptr || summary == nullptr || check == nullptr || B <= 0 || H <= 0 || N <= 0) return JVPFA_ERR_BAD_ARG;
+  *check = nullptr;
+  MaskCheck* c = take_mask_check();
+  if (c == nullptr) return JVPFA_ERR_LAUNCH;
+  *c->verdict = 0;
+  const int planes = (mask->stride[0] == 0 ? 1 : B) * (mask->stride[1] == 0 ? 1 : H);
+  const int n64 = (N + 63) / 64;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  mask_check_kernel<<<planes, 256, 0, s>>>(summary, n64 * n64, mask->kind, c->verdict);
+  if (cudaGetLastError() != cudaSuccess || cudaEventRecord(c->done, s) != cudaSuccess) {
+    free_mask_check(c);
+    return JVPFA_ERR_LAUNCH;
+  }
+  *check = c;
+  return JVPFA_OK;
+}
+
+int jvpfa_mask_check_end(void* check, int32_t* verdict) {
+  if (check == nullptr || verdict == nullptr) return JVPFA_ERR_BAD_ARG;
+  MaskCheck* c = static_cast<MaskCheck*>(check);
+  if (cudaEventSynchronize(c->done) != cudaSuccess) {
+    (void)cudaGetLastError();
+    free_mask_check(c);
+    return JVPFA_ERR_LAUNCH;
+  }
+  *verdict = *static_cast<volatile int*>(c->verdict);
+  give_back_mask_check(c);
+  return JVPFA_OK;
+}
+
 int jvpfa_fwd(const jvpfa_fwd_args* a, void* stream) {
+  return a == nullptr ? JVPFA_ERR_BAD_ARG : jvpfa_fwd_status(a, static_cast<int32_t*>(a->workspace), stream);
+}
+
+int jvpfa_fwd_status(const jvpfa_fwd_args* a, int32_t* status, void* stream) {
   if (a == nullptr) return JVPFA_ERR_BAD_ARG;
   int rc = check_common(a->B, a->H, a->N, a->D, a->dtype, a->causal, a->mask, a->workspace, a->workspace_bytes, kStatusBytes);
   if (rc != JVPFA_OK) return rc;
@@ -509,10 +614,10 @@ int jvpfa_fwd(const jvpfa_fwd_args* a, void* stream) {
       !(sm100_split_path_supported(a->dtype, a->D, a->N) && a->workspace_bytes >= fwd_sm100_split_workspace_bytes(*a)))
     return JVPFA_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (sm100_path_supported(a->dtype, a->D, a->N)) return launch_fwd_sm100(*a, s);
+  if (sm100_path_supported(a->dtype, a->D, a->N)) return launch_fwd_sm100(*a, status, s);
   // fp32: the tensor-core path when the workspace has room for the split operands, else the CUDA-core kernels
   if (sm100_split_path_supported(a->dtype, a->D, a->N) && a->workspace_bytes >= fwd_sm100_split_workspace_bytes(*a))
-    return launch_fwd_sm100_split(*a, s);
+    return launch_fwd_sm100_split(*a, status, s);
   {
     const jvpfa_strides* st[6] = {&a->q_strides, &a->k_strides, &a->v_strides, &a->tq_strides, &a->tk_strides, &a->tv_strides};
     for (int i = 0; i < (dual ? 6 : 3); ++i)
@@ -522,7 +627,7 @@ int jvpfa_fwd(const jvpfa_fwd_args* a, void* stream) {
 }
 
 namespace {
-int bwd_checked(const jvpfa_bwd_args* a, void* stream, void* const* events) {
+int bwd_checked(const jvpfa_bwd_args* a, int* status, void* stream, void* const* events) {
   if (a == nullptr) return JVPFA_ERR_BAD_ARG;
   // smallest workspace any path takes: the status block and one float4 of statistics per row
   int rc = check_common(a->B, a->H, a->N, a->D, a->dtype, a->causal, a->mask, a->workspace, a->workspace_bytes,
@@ -562,10 +667,10 @@ int bwd_checked(const jvpfa_bwd_args* a, void* stream, void* const* events) {
   LaunchMarks marks;
   marks.events = events;
   marks.stream = s;
-  if (sm100_path_supported(eff.dtype, eff.D, eff.N)) return launch_bwd_sm100(eff, s, marks);
+  if (sm100_path_supported(eff.dtype, eff.D, eff.N)) return launch_bwd_sm100(eff, status, s, marks);
   // fp32: the tensor-core path when the workspace has room for the split operands, else the CUDA-core kernels
   if (sm100_split_path_supported(eff.dtype, eff.D, eff.N) && eff.workspace_bytes >= bwd_sm100_split_workspace_bytes(eff))
-    return launch_bwd_sm100_split(eff, s, marks);
+    return launch_bwd_sm100_split(eff, status, s, marks);
   {
     const jvpfa_strides* st[8] = {&eff.q_strides, &eff.k_strides, &eff.v_strides, &eff.go_strides,
                                   &eff.tq_strides, &eff.tk_strides, &eff.tv_strides, &eff.gto_strides};
@@ -576,13 +681,19 @@ int bwd_checked(const jvpfa_bwd_args* a, void* stream, void* const* events) {
 }
 }  // namespace
 
-int jvpfa_bwd(const jvpfa_bwd_args* a, void* stream) { return bwd_checked(a, stream, nullptr); }
+int jvpfa_bwd(const jvpfa_bwd_args* a, void* stream) {
+  return a == nullptr ? JVPFA_ERR_BAD_ARG : bwd_checked(a, static_cast<int*>(a->workspace), stream, nullptr);
+}
+
+int jvpfa_bwd_status(const jvpfa_bwd_args* a, int32_t* status, void* stream) {
+  return a == nullptr ? JVPFA_ERR_BAD_ARG : bwd_checked(a, status, stream, nullptr);
+}
 
 int jvpfa_bwd_marked(const jvpfa_bwd_args* a, void* stream, void* const* events, int32_t n_events) {
   if (events == nullptr || n_events != 5) return JVPFA_ERR_BAD_ARG;
   for (int i = 0; i < 5; ++i)
     if (events[i] == nullptr) return JVPFA_ERR_BAD_ARG;
-  return bwd_checked(a, stream, events);
+  return a == nullptr ? JVPFA_ERR_BAD_ARG : bwd_checked(a, static_cast<int*>(a->workspace), stream, events);
 }
 
 int jvpfa_sm_clock_probe(float* mhz_out, int32_t duration_us, void* stream) {

@@ -63,6 +63,7 @@ inline MaskView make_mask_view(const jvpfa_mask& mask, const uint8_t* summary, i
 
 constexpr uint8_t kTileAnyKept = 1;     // some element of the tile takes part in attention
 constexpr uint8_t kTileAnyMasked = 2;   // some element needs the mask: a boolean False, or an additive entry that is not zero
+constexpr uint8_t kTileAnyNaN = 8;      // additive mask: some entry is a NaN (for the check of the mask; the kernels do not look at it)
 constexpr uint8_t kTileTwoValued = 4;   // additive mask: every entry is +-0 or the tile's one other value (bit words + tile values)
 
 #if defined(__CUDACC__)

@@ -17,9 +17,8 @@ taken with ``fwd_dual`` / ``dual``: the tangent output is part of the autograd g
 (``create_graph=True`` through these functions) is not supported and raises.
 
 Failure detection: every device-side wait in the kernels is bounded; one that gives up records a code in a status
-word and the kernel runs to its end. Each call enqueues a copy of that word to pinned host memory behind its
-kernels, and the next call on the same stream (without synchronising) or ``check()`` (which synchronises the
-device) raises ``_lib.JvpfaError`` with status ``ERR_DEVICE_TIMEOUT``; the results of the call that timed out are
+word in pinned host memory and the kernel runs to its end. The next call on the same stream (without synchronising) or
+``check()`` (which synchronises the device) raises ``_lib.JvpfaError`` with status ``ERR_DEVICE_TIMEOUT``; the results of the call that timed out are
 undefined. Errors the reference reports as Python exceptions (jvp_attention.py:2550, 2574, 3111) keep their types.
 """
 from __future__ import annotations
@@ -29,8 +28,6 @@ from typing import Optional
 import torch
 import torch.autograd.forward_ad as fwAD
 from torch import Tensor
-from torch.autograd import Function
-from torch.autograd.function import once_differentiable
 
 from . import _lib
 
@@ -82,6 +79,16 @@ def _draw_seed(dropout_p: float, dropout_seed) -> int:
     return int(torch.randint(0, 2 ** 63 - 1, (), dtype=torch.int64).item())
 
 
+def _mask_expandable(attn_mask: Optional[Tensor], q: Tensor) -> Optional[Tensor]:
+    """A mask that the native checks sent back and the Python checks let pass (unusual element type, unchecked shape)."""
+    if attn_mask is None:
+        return None
+    assert attn_mask.dim() == 4, "The provided attention mask must have 4 dimensions (Z, H, N_CTX, N_CTX)."
+    Z, H, N_CTX, _ = q.shape
+    attn_mask.expand(Z, H, N_CTX, N_CTX)
+    return _mask_for_kernel(attn_mask, q)
+
+
 def _mask_for_kernel(attn_mask: Optional[Tensor], q: Tensor) -> Optional[Tensor]:
     """Returns the mask in an element type the kernels read (bool, q.dtype-compatible or fp32)."""
     if attn_mask is None:
@@ -94,88 +101,19 @@ def _mask_for_kernel(attn_mask: Optional[Tensor], q: Tensor) -> Optional[Tensor]
     return m
 
 
-class _DualAttention(Function):
-    """(q, k, v, tq, tk, tv) -> (o, to, lse2, mu[, mask summary]); autograd through o and to."""
-
-    @staticmethod
-    def forward(q, k, v, tq, tk, tv, attn_mask, causal, sm_scale, dropout_p=0.0, dropout_seed=0):
-        B, H, N, D = q.shape
-        mask_c = _lib.make_mask(attn_mask, B, H, N)
-        summary = _lib.mask_summary(mask_c, attn_mask, B, H, N) if attn_mask is not None else None
-        o, to, lse2, mu = _lib.fwd(q, k, v, tq, tk, tv, mask_c, summary, causal, sm_scale, dropout_p, dropout_seed)
-        if summary is None:
-            summary = torch.empty(0, dtype=torch.uint8, device=q.device)
-        return o, to, lse2, mu, summary
-
-    @staticmethod
-    def setup_context(ctx, inputs, outputs):
-        q, k, v, tq, tk, tv, attn_mask, causal, sm_scale, dropout_p, dropout_seed = inputs
-        o, to, lse2, mu, summary = outputs
-        ctx.mark_non_differentiable(lse2, mu, summary)
-        ctx.save_for_backward(q, k, v, tq, tk, tv, o, to, lse2, mu, summary)
-        ctx.attn_mask = attn_mask
-        ctx.causal = causal
-        ctx.sm_scale = sm_scale
-        ctx.dropout = (dropout_p, dropout_seed)
-        ctx.set_materialize_grads(False)    # an output the loss does not use arrives as None, not as a tensor of zeros
-
-    @staticmethod
-    @once_differentiable      # the gradients come from kernels: differentiating them again raises instead of returning zeros
-    def backward(ctx, go, gto, _g_lse, _g_mu, _g_summary):
-        q, k, v, tq, tk, tv, o, to, lse2, mu, summary = ctx.saved_tensors
-        B, H, N, D = q.shape
-        if go is None and gto is None:
-            return (None,) * 11
-        mask_c = _lib.make_mask(ctx.attn_mask, B, H, N)
-        summ = summary if summary.numel() > 0 else None
-        if gto is None:
-            # Nothing flows back through the tangent output (a tangent that is only used as a detached target, or not at
-            # all): the primal-only backward -- what the reference's backward always is (jvp_attention.py:3081, 3226) --
-            # gives dq, dk, dv with half the tile products, and the tangent inputs get no gradient.
-            dq, dk, dv = _lib.bwd(q, k, v, None, None, None, o, None, lse2, mu, go, None, mask_c, summ, ctx.causal,
-                                  ctx.sm_scale, dropout_p=ctx.dropout[0], dropout_seed=ctx.dropout[1])
-            return dq, dk, dv, None, None, None, None, None, None, None, None
-        if go is None:
-            go = torch.zeros_like(o)
-        dq, dk, dv, dtq, dtk, dtv = _lib.bwd(q, k, v, tq, tk, tv, o, to, lse2, mu, go, gto, mask_c, summ,
-                                              ctx.causal, ctx.sm_scale, dropout_p=ctx.dropout[0], dropout_seed=ctx.dropout[1])
-        return dq, dk, dv, dtq, dtk, dtv, None, None, None, None, None
-
-
-class _PrimalAttention(Function):
-    """(q, k, v) -> (o, lse2): the primal-only entry; backward gives dq, dk, dv."""
-
-    @staticmethod
-    def forward(q, k, v, attn_mask, causal, sm_scale, dropout_p=0.0, dropout_seed=0):
-        B, H, N, D = q.shape
-        mask_c = _lib.make_mask(attn_mask, B, H, N)
-        summary = _lib.mask_summary(mask_c, attn_mask, B, H, N) if attn_mask is not None else None
-        o, _, lse2, mu = _lib.fwd(q, k, v, None, None, None, mask_c, summary, causal, sm_scale, dropout_p, dropout_seed)
-        if summary is None:
-            summary = torch.empty(0, dtype=torch.uint8, device=q.device)
-        return o, lse2, mu, summary
-
-    @staticmethod
-    def setup_context(ctx, inputs, outputs):
-        q, k, v, attn_mask, causal, sm_scale, dropout_p, dropout_seed = inputs
-        o, lse2, mu, summary = outputs
-        ctx.mark_non_differentiable(lse2, mu, summary)
-        ctx.save_for_backward(q, k, v, o, lse2, mu, summary)
-        ctx.attn_mask = attn_mask
-        ctx.causal = causal
-        ctx.sm_scale = sm_scale
-        ctx.dropout = (dropout_p, dropout_seed)
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, go, _g_lse, _g_mu, _g_summary):
-        q, k, v, o, lse2, mu, summary = ctx.saved_tensors
-        B, H, N, D = q.shape
-        mask_c = _lib.make_mask(ctx.attn_mask, B, H, N)
-        summ = summary if summary.numel() > 0 else None
-        dq, dk, dv = _lib.bwd(q, k, v, None, None, None, o, None, lse2, mu, go, None, mask_c, summ, ctx.causal,
-                              ctx.sm_scale, dropout_p=ctx.dropout[0], dropout_seed=ctx.dropout[1])
-        return dq, dk, dv, None, None, None, None, None
+def _call(q, k, v, attn_mask, dropout_p, causal, sm_scale, verify_attn_mask, dropout_seed, allow_dual):
+    """One native call (``csrc/host_torch.cpp``). It checks what an ordinary call has to satisfy and answers None when
+    something is unusual; the checks here then raise the exception that belongs to the mistake."""
+    if dropout_p != 0.0:
+        _validate(q, k, v, attn_mask, dropout_p, causal, False)
+        dropout_seed = _draw_seed(dropout_p, dropout_seed)
+    o = _lib.host().call(q, k, v, attn_mask, causal, sm_scale, dropout_p, dropout_seed or 0, verify_attn_mask, allow_dual)
+    if o is None:
+        _validate(q, k, v, attn_mask, dropout_p, causal, verify_attn_mask)
+        mask = _mask_expandable(attn_mask, q)
+        o = _lib.host().call(q, k, v, mask, causal, sm_scale, dropout_p, dropout_seed or 0, False, allow_dual)
+        assert o is not None, "q, k, v and the attention mask must be on one device"
+    return o
 
 
 class JVPAttn:
@@ -189,14 +127,7 @@ class JVPAttn:
         accepted for signature compatibility and ignored. ``dropout_p`` > 0 (every shape the tensor-core kernels take; the
         reference refuses it) drops attention probabilities with a pattern drawn from ``dropout_seed``, or from torch's
         CPU generator when no seed is given."""
-        _validate(q, k, v, attn_mask, dropout_p, causal, verify_attn_mask)
-        # strided views are read in place where the kernels can (``_lib.as_input``); the reference copies them (:2950)
-        q, k, v = (_lib.as_input(t) for t in (q, k, v))
-        if sm_scale is None:
-            sm_scale = q.shape[-1] ** -0.5
-        o, _, _, _ = _PrimalAttention.apply(q, k, v, _mask_for_kernel(attn_mask, q), bool(causal), float(sm_scale),
-                                            float(dropout_p), _draw_seed(dropout_p, dropout_seed))
-        return o
+        return _call(q, k, v, attn_mask, dropout_p, causal, sm_scale, verify_attn_mask, dropout_seed, False)
 
     @staticmethod
     def fwd_dual(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tensor | None = None, dropout_p: float = 0.0,
@@ -205,6 +136,8 @@ class JVPAttn:
         """Attention on forward-mode dual tensors (jvp_attention.py:2972-3063): works inside
         ``fwAD.dual_level()`` and under ``torch.func.jvp``; the result is a dual tensor whose tangent is
         the JVP. Inputs without a tangent contribute a zero tangent; if no input is dual this is ``fwd``."""
+        if not torch.compiler.is_compiling():
+            return _call(q, k, v, attn_mask, dropout_p, causal, sm_scale, verify_attn_mask, dropout_seed, True)
         q_p, q_t = fwAD.unpack_dual(q)
         k_p, k_t = fwAD.unpack_dual(k)
         v_p, v_t = fwAD.unpack_dual(v)
@@ -214,8 +147,8 @@ class JVPAttn:
         q_t = torch.zeros_like(q_p) if q_t is None else q_t
         k_t = torch.zeros_like(k_p) if k_t is None else k_t
         v_t = torch.zeros_like(v_p) if v_t is None else v_t
-        # ``dual`` validates, and inside torch.compile switches to the opaque operators (the reference routes its
-        # compiled dual call through its custom op in the same place, jvp_attention.py:3014-3041)
+        # inside torch.compile ``dual`` takes the opaque operators (the reference routes its compiled dual call through its
+        # custom op in the same place, jvp_attention.py:3014-3041)
         o, to = JVPAttn.dual(q_p, k_p, v_p, q_t, k_t, v_t, attn_mask=attn_mask, causal=causal, sm_scale=sm_scale,
                              verify_attn_mask=verify_attn_mask, dropout_p=dropout_p, dropout_seed=dropout_seed)
         return fwAD.make_dual(o, to)
@@ -237,14 +170,16 @@ class JVPAttn:
             o, to, _, _ = attn_fwd_dual(q, k, v, q_t, k_t, v_t, _mask_for_kernel(attn_mask, q), float(sm_scale),
                                         bool(causal), float(dropout_p), int(dropout_seed or 0))
             return o, to
-        _validate(q, k, v, attn_mask, dropout_p, causal, verify_attn_mask)
-        # strided views are read in place where the kernels can; the reference copies them (jvp_attention.py:3007)
-        q, k, v, q_t, k_t, v_t = (_lib.as_input(t) for t in (q, k, v, q_t, k_t, v_t))
-        if sm_scale is None:
-            sm_scale = q.shape[-1] ** -0.5
-        o, to, _, _, _ = _DualAttention.apply(q, k, v, q_t, k_t, v_t, _mask_for_kernel(attn_mask, q), bool(causal),
-                                              float(sm_scale), float(dropout_p), _draw_seed(dropout_p, dropout_seed))
-        return o, to
+        if dropout_p != 0.0:
+            _validate(q, k, v, attn_mask, dropout_p, causal, False)
+            dropout_seed = _draw_seed(dropout_p, dropout_seed)
+        out = _lib.host().dual(q, k, v, q_t, k_t, v_t, attn_mask, causal, sm_scale, dropout_p, dropout_seed or 0, verify_attn_mask)
+        if out is None:
+            _validate(q, k, v, attn_mask, dropout_p, causal, verify_attn_mask)
+            mask = _mask_expandable(attn_mask, q)
+            out = _lib.host().dual(q, k, v, q_t, k_t, v_t, mask, causal, sm_scale, dropout_p, dropout_seed or 0, False)
+            assert out is not None, "q, k, v, their tangents and the attention mask must share device, shape and dtype"
+        return out
 
 
 attention = JVPAttn.fwd

@@ -1,0 +1,51 @@
+"""The native host path on the GPU: the mask check that reads the mask's summary, and the tangent levels it takes."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwAD
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    assert torch.cuda.is_available()
+    return torch.device("cuda:0")
+
+
+@pytest.mark.parametrize("N", [33, 64, 130, 256])            # 33, 130: rows off the 16-byte grid (the generic summary kernel)
+@pytest.mark.parametrize("shape", ["per head", "per batch", "keys only"])
+def test_mask_check_verdicts(dev, N, shape):
+    """One plane of several with nothing kept, or one NaN in the last row and column, is an AssertionError; the mask before
+    that change is none; and the call after an error works."""
+    from jvp_flash_attention_b200 import attention
+    B, H = 3, 2
+    q = torch.randn(B, H, N, 64, device=dev, dtype=torch.float16)
+    full = {"per head": (B, H, N, N), "per batch": (B, 1, N, N), "keys only": (B, 1, 1, N)}[shape]
+    keep = torch.zeros(full, dtype=torch.bool, device=dev)
+    keep[..., -1, -1] = True                                  # a single kept entry per plane is enough
+    attention(q, q, q, attn_mask=keep)
+    keep[B - 1, -1] = False
+    with pytest.raises(AssertionError, match="all False"):
+        attention(q, q, q, attn_mask=keep)
+    attention(q, q, q, attn_mask=keep, verify_attn_mask=False)
+    for dtype in (torch.float16, torch.bfloat16, torch.float32):
+        bias = torch.full(full, float("-inf"), dtype=dtype, device=dev)   # excluded everywhere: not an error for a float mask
+        attention(q, q, q, attn_mask=bias)
+        bias[..., -1, -1][B - 1] = float("nan")
+        with pytest.raises(AssertionError, match="NaN"):
+            attention(q, q, q, attn_mask=bias)
+
+
+def test_tangents_that_cannot_be_taken_raise(dev):
+    """``fwd`` and ``dual`` on dual tensors, and a second level of tangents, raise instead of dropping a tangent."""
+    from jvp_flash_attention_b200.jvp_attention import JVPAttn, attention
+    q, t = (torch.randn(1, 1, 64, 64, device=dev, dtype=torch.float16) for _ in range(2))
+    with fwAD.dual_level():
+        d = fwAD.make_dual(q, t)
+        with pytest.raises(RuntimeError):
+            attention(d, q, q)
+        with pytest.raises(RuntimeError):
+            JVPAttn.dual(d, q, q, t, t, t)
+    inner = lambda x: torch.func.jvp(lambda y: JVPAttn.fwd_dual(y, q, q), (x,), (t,))[1]
+    with pytest.raises(RuntimeError):
+        torch.func.jvp(inner, (q,), (t,))
