@@ -58,7 +58,7 @@ def _build_host() -> None:
 def build(force: bool = False, verbose: bool = False) -> Path:
     nvcc = _nvcc()
     OBJ.mkdir(parents=True, exist_ok=True)
-    srcs = sorted(CSRC.glob("*.cu"))
+    srcs = sorted(CSRC.glob("*.cu"), key=lambda f: ("bwd" not in f.name, f.name))      # the long compilations first
     hdr_m = _newest_header_mtime()
     jobs = []
     for src in srcs:
@@ -72,13 +72,17 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         return src, r
 
-    with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
+    host_stale = force or not HOST_LIB.exists() or HOST_LIB.stat().st_mtime < max(HOST_SRC.stat().st_mtime, hdr_m)
+    with ThreadPoolExecutor(max_workers=min(8, len(jobs) + 1)) as ex:
+        host_job = ex.submit(_build_host) if host_stale else None
         for src, r in ex.map(compile_one, jobs):
             if verbose or r.returncode != 0:
                 sys.stderr.write(f"--- {src.name}\n{r.stdout}{r.stderr}\n")
             (OBJ / (src.stem + ".ptxas.txt")).write_text(r.stderr)
             if r.returncode != 0:
                 raise RuntimeError(f"nvcc failed on {src.name}")
+        if host_job is not None:
+            host_job.result()
     objs = [str(OBJ / (s.stem + ".o")) for s in srcs]
     if jobs or not LIB.exists() or force:
         cmd = [nvcc, "-shared", "-o", str(LIB), *objs, "-gencode", "arch=compute_100a,code=sm_100a"]
@@ -86,8 +90,6 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
-    if force or not HOST_LIB.exists() or HOST_LIB.stat().st_mtime < max(HOST_SRC.stat().st_mtime, hdr_m):
-        _build_host()
     return LIB
 
 

@@ -98,10 +98,18 @@ int launch_fwd_sm100_split(const jvpfa_fwd_args& a, int* status, cudaStream_t st
 int launch_bwd_sm100_split(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks);
 
 int launch_fwd_sm100(const jvpfa_fwd_args& a, int* status, cudaStream_t stream);
+int launch_fwd_sm100_d64(const jvpfa_fwd_args& a, int* status, cudaStream_t stream);
+int launch_fwd_sm100_d128(const jvpfa_fwd_args& a, int* status, cudaStream_t stream);
+int launch_fwd_sm100_d256(const jvpfa_fwd_args& a, int* status, cudaStream_t stream);
 int launch_bwd_sm100(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks);
+int launch_bwd_sm100_d64_bf16(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks);
+int launch_bwd_sm100_d64_fp16(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks);
+int launch_bwd_sm100_d128_bf16(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks);
+int launch_bwd_sm100_d128_fp16(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks);
+int launch_bwd_sm100_d256(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks);
 size_t bwd_sm100_workspace_bytes(const jvpfa_bwd_args& a);
 bool sm100_path_supported(int dtype, int D, int N);
-inline int sm100_padded_dim(int D) { return D <= 64 ? 64 : 128; }
+bool sm100_wide_path_supported(int dtype, int D, int N);   // 16-bit inputs, head dimensions 136 to 256; no dropout
 
 int launch_fwd_generic(const jvpfa_fwd_args& a, cudaStream_t stream);
 int launch_bwd_generic(const jvpfa_bwd_args& a, cudaStream_t stream, const LaunchMarks& marks);

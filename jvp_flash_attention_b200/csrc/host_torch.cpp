@@ -113,7 +113,7 @@ int dtype_code(at::ScalarType t) {
 // (dtype, head dimension) that the tensor-core kernels take; they read strided inputs in place
 bool tensor_core_path(at::ScalarType t, int64_t D) {
   if (D < 8 || D % 8 != 0) return false;
-  return t == at::kFloat ? D <= 64 : D <= 128;
+  return t == at::kFloat ? D <= 64 : D <= 256;
 }
 
 // Readable in place: last axis contiguous, every other stride (of an axis longer than 1) positive and a multiple of 16 bytes,

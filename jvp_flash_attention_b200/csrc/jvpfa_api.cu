@@ -467,7 +467,7 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 // Input layouts: the tensor-core paths read strided views in place when TMA (16-bit inputs) or the split pre-pass
 // (fp32 inputs) can address them; the CUDA-core kernels take contiguous tensors only.
 int check_layouts(const void* const* ptrs, const jvpfa_strides* const* strides, int n, int B, int H, int N, int D, int dtype) {
-  const bool tensor_cores = sm100_path_supported(dtype, D, N) || sm100_split_path_supported(dtype, D, N);
+  const bool tensor_cores = sm100_path_supported(dtype, D, N) || sm100_wide_path_supported(dtype, D, N) || sm100_split_path_supported(dtype, D, N);
   const int elem = dtype == JVPFA_F32 ? 4 : 2;
   for (int i = 0; i < n; ++i) {
     if (ptrs[i] == nullptr || is_contiguous(*strides[i], H, N, D)) continue;
@@ -614,7 +614,7 @@ int jvpfa_fwd_status(const jvpfa_fwd_args* a, int32_t* status, void* stream) {
       !(sm100_split_path_supported(a->dtype, a->D, a->N) && a->workspace_bytes >= fwd_sm100_split_workspace_bytes(*a)))
     return JVPFA_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (sm100_path_supported(a->dtype, a->D, a->N)) return launch_fwd_sm100(*a, status, s);
+  if (sm100_path_supported(a->dtype, a->D, a->N) || sm100_wide_path_supported(a->dtype, a->D, a->N)) return launch_fwd_sm100(*a, status, s);
   // fp32: the tensor-core path when the workspace has room for the split operands, else the CUDA-core kernels
   if (sm100_split_path_supported(a->dtype, a->D, a->N) && a->workspace_bytes >= fwd_sm100_split_workspace_bytes(*a))
     return launch_fwd_sm100_split(*a, status, s);
@@ -667,7 +667,7 @@ int bwd_checked(const jvpfa_bwd_args* a, int* status, void* stream, void* const*
   LaunchMarks marks;
   marks.events = events;
   marks.stream = s;
-  if (sm100_path_supported(eff.dtype, eff.D, eff.N)) return launch_bwd_sm100(eff, status, s, marks);
+  if (sm100_path_supported(eff.dtype, eff.D, eff.N) || sm100_wide_path_supported(eff.dtype, eff.D, eff.N)) return launch_bwd_sm100(eff, status, s, marks);
   // fp32: the tensor-core path when the workspace has room for the split operands, else the CUDA-core kernels
   if (sm100_split_path_supported(eff.dtype, eff.D, eff.N) && eff.workspace_bytes >= bwd_sm100_split_workspace_bytes(eff))
     return launch_bwd_sm100_split(eff, status, s, marks);
