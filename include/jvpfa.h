@@ -49,7 +49,7 @@ typedef struct jvpfa_mask {
  * contiguous layout (H*N*D, N*D, D). A strided input (for instance q = qkv.permute(2,0,3,1,4)[0] of a fused projection,
  * or an upstream gradient that is a transposed view) is read in place by the tensor-core kernels when every stride
  * is a multiple of 16 bytes and the pointer is 16-byte aligned; otherwise, and for the shapes that run on the
- * CUDA-core kernels (head dimension above 128 or not a multiple of 8; fp32 above 64), the call returns
+ * CUDA-core kernels (head dimension above 256 or not a multiple of 8; fp32 above 64), the call returns
  * JVPFA_ERR_UNSUPPORTED and the caller copies the tensor first. */
 typedef struct jvpfa_strides {
   int64_t b, h, n;

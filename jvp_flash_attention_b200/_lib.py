@@ -193,7 +193,7 @@ def _ptr(t):
 def tensor_core_path(dtype: torch.dtype, D: int) -> bool:
     """Whether (dtype, head dimension) runs on the tensor-core kernels, which read strided inputs in place."""
     if dtype in (torch.float16, torch.bfloat16):
-        return 8 <= D <= 128 and D % 8 == 0
+        return 8 <= D <= 256 and D % 8 == 0
     return dtype == torch.float32 and 8 <= D <= 64 and D % 8 == 0
 
 
@@ -369,7 +369,7 @@ def mask_summary(mask_c: Mask, mask_tensor, B, H, N):
 def dropout_supported(dtype: torch.dtype, D: int) -> bool:
     """Dropout runs in the tensor-core kernels: fp16 / bf16 with a head dimension that is a multiple of 8 up to 128, fp32
     up to 64."""
-    return tensor_core_path(dtype, D)
+    return tensor_core_path(dtype, D) and D <= 128
 
 
 def fwd(q, k, v, tq, tk, tv, mask_c: Mask, summary, causal: bool, sm_scale: float, dropout_p: float = 0.0,

@@ -110,6 +110,10 @@ struct FwdCfg {
 // one score row, 32 columns; the row maximum and the final row sums are exchanged through shared
 // memory); warps 8, 11: TMA producers (one lane each: Q and K pairs / V tiles); warps 9, 10: MMA issuers (one lane each: scores / outputs), warp 9 owns the
 // TMEM allocation.
+// D = 256 (head dimensions 136 to 256): O and T alone would fill TMEM, so two CTAs share a query tile, each with half of
+// the output columns (V, tV columns) and all of the score products: 9 tile products where one CTA would run 6. Q, tQ take
+// 128 KB of shared memory; K, tK go through four 16 KB slots by 64-column slab, V, tV have one 32 KB buffer.
+// B=2 H=8 N=1024 D=256 causal fp16: 0.063 ms (3.11 ms on the CUDA cores).
 // PAD: the tensors' head dimension is smaller than D (columns beyond it are zero-filled by TMA); the K steps and
 // output columns that would only see zeros are then skipped at run time.
 // DROP: dropout on the attention probabilities (dropout.cuh): P and W reach TMEM dropped out and rescaled, the row sums l

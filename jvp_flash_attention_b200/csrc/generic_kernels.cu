@@ -1,5 +1,6 @@
-// CUDA-core (fp32 FMA) kernels for the shapes the tensor-core kernels do not take: fp32 inputs
-// (which must meet a 1e-4 tolerance that TF32 cannot) and head dimensions other than 64 / 128.
+// CUDA-core (fp32 FMA) kernels for the shapes the tensor-core kernels do not take: head dimensions that are not a multiple
+// of 8, fp32 inputs with a head dimension above 64 (which must meet a 1e-4 tolerance that TF32 cannot), and fp32 calls
+// whose workspace has no room for the split operands.
 // Same mathematics and the same three-family split as the tensor-core kernels, 32x32 score tiles,
 // all operands staged in shared memory as fp32, transposed ([d][row], row pitch 33) so that both
 // the score products and the output products read shared memory without bank conflicts.
