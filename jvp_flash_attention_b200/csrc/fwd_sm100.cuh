@@ -671,6 +671,24 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 9) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
+template <bool BF16>
+FwdKParams make_fwd_params(const jvpfa_fwd_args& a, int* status) {
+  FwdKParams p{};
+  p.H = a.H; p.N = a.N; p.D = a.D; p.causal = a.causal;
+  p.s = a.sm_scale;
+  p.c1 = a.sm_scale * 1.4426950408889634f;
+  p.thresh = BF16 ? 8.0f : 6.0f;
+  p.mv = make_mask_view(a.mask, a.mask_summary, a.B, a.H, a.N);
+  p.o = a.o; p.to = a.to; p.lse2 = a.lse2; p.mu = a.mu;
+  p.status = status;
+  p.budget_ns = wait_budget_ns();
+  p.drop = make_dropout_params(a.dropout_p, a.dropout_seed);
+  p.n_qt = (a.N + 127) / 128;
+  p.n_units = a.B * a.H;
+  p.unit_group = unit_group_size(p.n_units);
+  return p;
+}
+
 template <int D, bool DUAL, bool BF16, bool PAD, bool DROP = false>
 int launch_one(const jvpfa_fwd_args& a, int* status, cudaStream_t stream) {
   using C = FwdCfg<D>;
@@ -689,23 +707,11 @@ int launch_one(const jvpfa_fwd_args& a, int* status, cudaStream_t stream) {
     mTQ = mQ; mTK = mK; mTV = mV;
   }
   if (!ok) return JVPFA_ERR_LAUNCH;
-  FwdKParams p{};
-  p.H = a.H; p.N = a.N; p.D = a.D; p.causal = a.causal;
-  p.s = a.sm_scale;
-  p.c1 = a.sm_scale * 1.4426950408889634f;
-  p.thresh = BF16 ? 8.0f : 6.0f;
-  p.mv = make_mask_view(a.mask, a.mask_summary, a.B, a.H, a.N);
-  p.o = a.o; p.to = a.to; p.lse2 = a.lse2; p.mu = a.mu;
-  p.status = status;
-  p.budget_ns = wait_budget_ns();
-  p.drop = make_dropout_params(a.dropout_p, a.dropout_seed);
+  const FwdKParams p = make_fwd_params<BF16>(a, status);
   auto kern = fwd_sm100_kernel<D, DUAL, BF16, PAD, false, DROP>;
   const size_t smem = C::smem_bytes();
   static SmemOptIn opt_in;
   if (!opt_in.set(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_LAUNCH;
-  p.n_qt = (a.N + C::BM - 1) / C::BM;
-  p.n_units = a.B * a.H;
-  p.unit_group = unit_group_size(p.n_units);
   dim3 grid(static_cast<unsigned>(p.n_qt) * static_cast<unsigned>(p.n_units) * (C::WIDE ? 2u : 1u));
   kern<<<grid, 384, smem, stream>>>(mQ, mTQ, mK, mTK, mV, mTV, p);
   return cudaGetLastError() == cudaSuccess ? JVPFA_OK : JVPFA_ERR_LAUNCH;
@@ -741,23 +747,11 @@ int launch_split(const jvpfa_fwd_args& a, int* status, cudaStream_t stream) {
     mTQ = mQ; mTK = mK; mTV = mV;
   }
   if (!ok) return JVPFA_ERR_LAUNCH;
-  FwdKParams p{};
-  p.H = a.H; p.N = a.N; p.D = a.D; p.causal = a.causal;
-  p.s = a.sm_scale;
-  p.c1 = a.sm_scale * 1.4426950408889634f;
-  p.thresh = 8.0f;
-  p.mv = make_mask_view(a.mask, a.mask_summary, a.B, a.H, a.N);
-  p.o = a.o; p.to = a.to; p.lse2 = a.lse2; p.mu = a.mu;
-  p.status = status;
-  p.budget_ns = wait_budget_ns();
-  p.drop = make_dropout_params(a.dropout_p, a.dropout_seed);
+  const FwdKParams p = make_fwd_params<true>(a, status);
   auto kern = fwd_sm100_kernel<128, DUAL, true, false, true, DROP>;
   const size_t smem = C::smem_bytes();
   static SmemOptIn opt_in;
   if (!opt_in.set(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_LAUNCH;
-  p.n_qt = (a.N + C::BM - 1) / C::BM;
-  p.n_units = a.B * a.H;
-  p.unit_group = unit_group_size(p.n_units);
   dim3 grid(static_cast<unsigned>(p.n_qt) * static_cast<unsigned>(p.n_units));
   kern<<<grid, 384, smem, stream>>>(mQ, mTQ, mK, mTK, mV, mTV, p);
   return cudaGetLastError() == cudaSuccess ? JVPFA_OK : JVPFA_ERR_LAUNCH;
