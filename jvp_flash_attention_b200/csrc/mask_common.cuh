@@ -112,6 +112,14 @@ __device__ __forceinline__ void mask_apply_bits(float2 (&x2)[16], uint32_t mb, f
   }
 }
 
+// The mask as the thread that owns query row q sees the 64 keys of a tile: how it is applied (mask_tile_mode), and for mode 1
+// the two words and what a zero bit adds. Fetched a tile ahead of its use; nothing for a tile at or beyond n_tiles.
+struct MaskRow {
+  int mode;
+  float other;
+  uint32_t bits[2];
+};
+
 __device__ __forceinline__ float mask_elem_as_float(const void* base, int64_t idx, int dtype) {
   if (dtype == JVPFA_F32) return static_cast<const float*>(base)[idx];
   if (dtype == JVPFA_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(base)[idx]);
@@ -182,6 +190,86 @@ __device__ __forceinline__ void mask_bias_run(float (&bias)[CNT], const MaskView
       for (int i = 0; i < CNT; ++i)
         bias[i] = (first + i < N) ? mask_elem_as_float(mv.ptr, base + i * step, mv.dtype) * kLog2e : ninf;
     }
+  }
+}
+
+__device__ __forceinline__ MaskRow mask_row_of(const MaskView& mv, int b, int h, int q, int tile, int n_tiles) {
+  MaskRow r;
+  r.mode = 0;
+  r.other = -INFINITY;
+  r.bits[0] = r.bits[1] = 0xFFFFFFFFu;
+  if (mv.kind == JVPFA_MASK_NONE || tile >= n_tiles) return r;
+  r.mode = mask_tile_mode(mv, mask_tile_bits(mv, b, h, q >> 6, tile));
+  if (mv.rowbits != nullptr) {      // (loaded whatever the mode is: its load does not wait for the tile's flags)
+    const int64_t plane = static_cast<int64_t>(mv.s0 == 0 ? 0 : b) * mv.Hm + (mv.s1 == 0 ? 0 : h);
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(mv.rowbits) + (plane * mv.n64 + tile) * mv.n_pad + q);
+    r.bits[0] = v.x;
+    r.bits[1] = v.y;
+    if (mv.kind == JVPFA_MASK_ADDITIVE) r.other = mask_tile_value(mv, b, h, q >> 6, tile) * 1.4426950408889634f;
+  }
+  return r;
+}
+
+// The same for the thread that owns key row k, against the 64 queries of query tile `tile`.
+__device__ __forceinline__ MaskRow mask_col_of(const MaskView& mv, int b, int h, int tile, int k, int n_tiles) {
+  MaskRow r;
+  r.mode = 0;
+  r.other = -INFINITY;
+  r.bits[0] = r.bits[1] = 0xFFFFFFFFu;
+  if (mv.kind == JVPFA_MASK_NONE || tile >= n_tiles) return r;
+  r.mode = mask_tile_mode(mv, mask_tile_bits(mv, b, h, tile, k >> 6));
+  if (mv.colbits != nullptr) {
+    const int64_t plane = static_cast<int64_t>(mv.s0 == 0 ? 0 : b) * mv.Hm + (mv.s1 == 0 ? 0 : h);
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(mv.colbits) + (plane * mv.n64 + tile) * mv.n_pad + k);
+    r.bits[0] = v.x;
+    r.bits[1] = v.y;
+    if (mv.kind == JVPFA_MASK_ADDITIVE) r.other = mask_tile_value(mv, b, h, tile, k >> 6) * 1.4426950408889634f;
+  }
+  return r;
+}
+
+// x2 += the additive (or boolean) mask's entries (q, k0 .. k0 + 63) in the log2 domain, read element by element. A row of
+// 16-bit entries that is contiguous and aligned is loaded whole before any of it is used; the rest goes 16 entries at a time.
+__device__ __forceinline__ void mask_add_row64(float2 (&x2)[2][16], const MaskView& mv, int b, int h, int q, int k0, int N) {
+  const int64_t base = b * mv.s0 + h * mv.s1 + static_cast<int64_t>(q) * mv.s2 + static_cast<int64_t>(k0) * mv.s3;
+  const uint8_t* mp = static_cast<const uint8_t*>(mv.ptr) + base * 2;
+  if (mv.kind == JVPFA_MASK_ADDITIVE && mv.dtype != JVPFA_F32 && mv.s3 == 1 && k0 + 64 <= N && (reinterpret_cast<uintptr_t>(mp) & 15) == 0) {
+    uint4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(mp) + i);
+    const float2 l2e = make_float2(1.4426950408889634f, 1.4426950408889634f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        float2 f;
+        if (mv.dtype == JVPFA_BF16) f = make_float2(__uint_as_float(u[c] << 16), __uint_as_float(u[c] & 0xFFFF0000u));
+        else f = __half22float2(*reinterpret_cast<const __half2*>(&u[c]));
+        float2& x = x2[i >> 2][(i & 3) * 4 + c];
+        x = __ffma2_rn(f, l2e, x);
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    float bias[16];
+    mask_bias_run<16>(bias, mv, b, h, q, k0 + 16 * c, N, true);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x2[c >> 1][8 * (c & 1) + i] = __fadd2_rn(x2[c >> 1][8 * (c & 1) + i], make_float2(bias[2 * i], bias[2 * i + 1]));
+  }
+}
+
+// x2 += the mask's entries (q0 .. q0 + 63, k) in the log2 domain, element by element down a column. Neighbouring lanes own
+// neighbouring keys, so a warp's loads are row segments; 32 of them are in flight before the first is used.
+__device__ __forceinline__ void mask_add_col64(float2 (&x2)[2][16], const MaskView& mv, int b, int h, int q0, int k, int N) {
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    float bias[32];
+    mask_bias_run<32>(bias, mv, b, h, q0 + 32 * c, k, N, false);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x2[c][i] = __fadd2_rn(x2[c][i], make_float2(bias[2 * i], bias[2 * i + 1]));
   }
 }
 #endif
