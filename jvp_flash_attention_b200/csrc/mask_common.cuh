@@ -210,24 +210,6 @@ __device__ __forceinline__ MaskRow mask_row_of(const MaskView& mv, int b, int h,
   return r;
 }
 
-// The same for the thread that owns key row k, against the 64 queries of query tile `tile`.
-__device__ __forceinline__ MaskRow mask_col_of(const MaskView& mv, int b, int h, int tile, int k, int n_tiles) {
-  MaskRow r;
-  r.mode = 0;
-  r.other = -INFINITY;
-  r.bits[0] = r.bits[1] = 0xFFFFFFFFu;
-  if (mv.kind == JVPFA_MASK_NONE || tile >= n_tiles) return r;
-  r.mode = mask_tile_mode(mv, mask_tile_bits(mv, b, h, tile, k >> 6));
-  if (mv.colbits != nullptr) {
-    const int64_t plane = static_cast<int64_t>(mv.s0 == 0 ? 0 : b) * mv.Hm + (mv.s1 == 0 ? 0 : h);
-    const uint2 v = __ldg(reinterpret_cast<const uint2*>(mv.colbits) + (plane * mv.n64 + tile) * mv.n_pad + k);
-    r.bits[0] = v.x;
-    r.bits[1] = v.y;
-    if (mv.kind == JVPFA_MASK_ADDITIVE) r.other = mask_tile_value(mv, b, h, tile, k >> 6) * 1.4426950408889634f;
-  }
-  return r;
-}
-
 // x2 += the additive (or boolean) mask's entries (q, k0 .. k0 + 63) in the log2 domain, read element by element. A row of
 // 16-bit entries that is contiguous and aligned is loaded whole before any of it is used; the rest goes 16 entries at a time.
 __device__ __forceinline__ void mask_add_row64(float2 (&x2)[2][16], const MaskView& mv, int b, int h, int q, int k0, int N) {
@@ -258,18 +240,6 @@ __device__ __forceinline__ void mask_add_row64(float2 (&x2)[2][16], const MaskVi
     mask_bias_run<16>(bias, mv, b, h, q, k0 + 16 * c, N, true);
 #pragma unroll
     for (int i = 0; i < 8; ++i) x2[c >> 1][8 * (c & 1) + i] = __fadd2_rn(x2[c >> 1][8 * (c & 1) + i], make_float2(bias[2 * i], bias[2 * i + 1]));
-  }
-}
-
-// x2 += the mask's entries (q0 .. q0 + 63, k) in the log2 domain, element by element down a column. Neighbouring lanes own
-// neighbouring keys, so a warp's loads are row segments; 32 of them are in flight before the first is used.
-__device__ __forceinline__ void mask_add_col64(float2 (&x2)[2][16], const MaskView& mv, int b, int h, int q0, int k, int N) {
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    float bias[32];
-    mask_bias_run<32>(bias, mv, b, h, q0 + 32 * c, k, N, false);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) x2[c][i] = __fadd2_rn(x2[c][i], make_float2(bias[2 * i], bias[2 * i + 1]));
   }
 }
 #endif
