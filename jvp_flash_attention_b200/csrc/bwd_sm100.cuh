@@ -6,7 +6,7 @@
 // gradient through the tangent output and the tangent-input gradients, which the reference does
 // not compute (jvp_attention.py:3081, 3226).
 //
-// One kernel template, one instantiation per output family. A CTA owns a "row" tile of 128 sequence positions
+// One device function template, one instantiation per output family; a launch holds all families. A CTA owns a "row" tile of 128 sequence positions
 // whose operands stay in shared memory, and streams 64-wide "column" tiles of the other side:
 //   family Q : rows = queries.  scores S, tS, X, A (q on TMEM lanes)    -> dQ, dtQ
 //   family K : rows = keys.     transposed scores (k on TMEM lanes)      -> dK, dtK
@@ -46,19 +46,16 @@ enum { FAM_Q = 0, FAM_K = 1, FAM_V = 2, FAM_KV = 3 };
 
 struct BwdKParams {
   int H, N;
-  int n_rt, n_units;   // row tiles per (batch, head) unit, number of units: the grid has n_rt * n_units blocks
+  int first_fam;       // first family of the launch (an index into BwdFamilies::FAM)
+  int n_rt, n_units;   // row tiles per (batch, head) unit, number of units: n_rt * n_units blocks per family
   int unit_group;      // units per group of the block order
   int D;     // head dimension of the tensors (the kernel is compiled for it rounded up to 64 or 128)
   int causal;
   float c1;  // sm_scale * log2(e)
   float s;   // sm_scale
-  float out_scale;
   MaskView mv;
   const float4* stats;  // per (b,h,q): lse2, mu, Delta, a
-  void* out0;
-  void* out1;
-  void* out2;   // family KV: dV, dtV (written unscaled)
-  void* out3;
+  void *dq, *dtq, *dk, *dtk, *dv, *dtv;
   int* status;
   uint64_t budget_ns;
   DropoutParams drop;
@@ -85,6 +82,30 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 __device__ __forceinline__ uint32_t pack2_residual(float a, float b, uint32_t hi) {
   return pack2<true>(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xFFFF0000u));
 }
+
+// The tensor maps of a backward call, one with the row-side and one with the column-side box per operand: every operand
+// is row-side in one family and column-side in another, so they are encoded once for all launches of the call.
+enum { OP_Q = 0, OP_K, OP_V, OP_GO, OP_TQ, OP_TK, OP_TV, OP_GTO, N_OPS };
+struct BwdMaps {
+  CUtensorMap row[N_OPS], col[N_OPS];
+  bool encode(const jvpfa_bwd_args& a) {
+    const void* const ptr[N_OPS] = {a.q, a.k, a.v, a.go, a.tq, a.tk, a.tv, a.gto};
+    const jvpfa_strides* const st[N_OPS] = {&a.q_strides, &a.k_strides, &a.v_strides, &a.go_strides,
+                                            &a.tq_strides, &a.tk_strides, &a.tv_strides, &a.gto_strides};
+    const bool dual = a.tq != nullptr;
+    for (int i = 0; i < N_OPS; ++i) {
+      if (!dual && i >= OP_TQ) {   // tangent operands of a primal-only call: aliases, never used
+        row[i] = row[i - OP_TQ];
+        col[i] = col[i - OP_TQ];
+        continue;
+      }
+      const TensorView v = make_view(ptr[i], *st[i], a.H, a.N, a.D);
+      if (!make_tile_map(&row[i], v, a.B, a.H, a.N, a.D, 128, a.dtype) || !make_tile_map(&col[i], v, a.B, a.H, a.N, a.D, 64, a.dtype))
+        return false;
+    }
+    return true;
+  }
+};
 
 // SPLIT: fp32 inputs on the tensor cores. The operands arrive as rows of 128 bf16 numbers [hi(64) | lo(64)] written by the
 // split pre-pass, so the tiles have the geometry of the D = 128 kernel with the hi parts in slab 0 and the lo parts in
@@ -117,8 +138,8 @@ struct BwdCfg {
   static constexpr size_t smem_bytes() { return NR * TILE_R + (NA + NB) * PAIR + 2 * BC * 16 + (NBAR + 2) * 8; }
 };
 
-// Tensor maps: rmK = row-side operands (box of 128 rows, all slabs); cmK = column-side operands (box of
-// 64 rows, one 64-column slab), cm0/cm1 the first pair, cm2/cm3 the second pair:
+// Operands: rmK = row-side (box of 128 rows, all slabs); cmK = column-side (box of 64 rows, one 64-column slab), cm0/cm1 the
+// first pair, cm2/cm3 the second pair:
 //  family Q: rm = Q, tQ, gO, gtO;  first pair (K, tK),  second pair (V, tV)
 //  family K: rm = K, tK, V, tV;    first pair (Q, tQ),  second pair (gO, gtO)
 //  family V: rm = K, tK;           first pair (Q, tQ),  second pair (gO, gtO)
@@ -139,21 +160,21 @@ struct BwdCfg {
 // regenerated here: it scales X and A (the gradients that arrive through V, tV) in families Q, K, and P, tP (the operands
 // of dV, dtV) in family V; Delta and a come from the dropped-out O, tO and need no change.
 template <int D, int FAM, bool BF16, bool PAD, bool DUAL, bool SPLIT = false, bool DROP = false>
-__global__ void __launch_bounds__(352, 1)
-bwd_sm100_kernel(const __grid_constant__ CUtensorMap rm0, const __grid_constant__ CUtensorMap rm1,
-                 const __grid_constant__ CUtensorMap rm2, const __grid_constant__ CUtensorMap rm3,
-                 const __grid_constant__ CUtensorMap cm0, const __grid_constant__ CUtensorMap cm1,
-                 const __grid_constant__ CUtensorMap cm2, const __grid_constant__ CUtensorMap cm3,
-                 const BwdKParams p) {
+__device__ __forceinline__ void bwd_family(const BwdMaps& maps, const BwdKParams& p, const int rt, const int bh, uint8_t* smem) {
   using C = BwdCfg<D, FAM, SPLIT>;
   constexpr int NA = C::NA, NB = C::NB;
   constexpr int SLABS = D / 64;
   constexpr int DV = C::DV;
   static_assert(!SPLIT || (D == 128 && BF16 && !PAD), "the split-fp32 mode runs on the 128-column geometry in bf16");
 
+  constexpr bool ROWS_Q = FAM == FAM_Q;
+  const CUtensorMap &rm0 = maps.row[ROWS_Q ? OP_Q : OP_K], &rm1 = maps.row[ROWS_Q ? OP_TQ : OP_TK],
+                    &rm2 = maps.row[ROWS_Q ? OP_GO : OP_V], &rm3 = maps.row[ROWS_Q ? OP_GTO : OP_TV],
+                    &cm0 = maps.col[ROWS_Q ? OP_K : OP_Q], &cm1 = maps.col[ROWS_Q ? OP_TK : OP_TQ],
+                    &cm2 = maps.col[ROWS_Q ? OP_V : OP_GO], &cm3 = maps.col[ROWS_Q ? OP_TV : OP_GTO];
+
   // Everything lives in dynamic shared memory so that the 128-byte-swizzled tiles can start at its
   // 1024-byte-aligned base without alignment slack: tiles, then statistics, then barriers.
-  extern __shared__ __align__(1024) uint8_t smem[];
   auto sR = [&](int i) { return smem + i * C::TILE_R; };
   auto sA = [&](int k) { return smem + C::NR * C::TILE_R + k * C::PAIR; };
   auto sB = [&](int k) { return smem + C::NR * C::TILE_R + (NA + k) * C::PAIR; };
@@ -186,11 +207,6 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap rm0, const __grid_constant_
   }
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_rt = p.n_rt;
-  // heavier tiles first under a causal mask: late query tiles, early key tiles
-  const BlockWork work = block_work(blockIdx.x, n_rt, p.n_units, p.unit_group, p.causal && FAM == FAM_Q);
-  const int rt = work.tile;
-  const int bh = work.unit;
   const int b = bh / p.H, h = bh % p.H;
   const int r0 = rt * C::BR;
   const int N = p.N;
@@ -799,7 +815,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap rm0, const __grid_constant_
       mbar_wait(&r_full, 0, w, 36);
       if constexpr (C::NR == 4) mbar_wait(&r23_full, 0, w, 38);
     }
+    void* const out0 = FAM == FAM_Q ? p.dq : (FAM == FAM_V ? p.dv : p.dk);
+    void* const out1 = FAM == FAM_Q ? p.dtq : (FAM == FAM_V ? p.dtv : p.dtk);
     if constexpr (SPLIT) {
+      const float scale = FAM == FAM_V ? 1.0f : p.s;
       // fp32 outputs: this warpgroup's 32 columns are 128 bytes per row
       uint8_t* patch = sR(0) + warp * (32 * 128);
       uint32_t q0[2][16], q1[2][16];
@@ -815,18 +834,18 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap rm0, const __grid_constant_
         }
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          q0[i >> 4][i & 15] = __float_as_uint(__uint_as_float(a0[i]) * p.out_scale);
-          if constexpr (DUAL) q1[i >> 4][i & 15] = __float_as_uint(__uint_as_float(a1[i]) * p.out_scale);
+          q0[i >> 4][i & 15] = __float_as_uint(__uint_as_float(a0[i]) * scale);
+          if constexpr (DUAL) q1[i >> 4][i & 15] = __float_as_uint(__uint_as_float(a1[i]) * scale);
         }
       }
       const int col0 = wg * 32;
       const int wrow0 = r0 + (warp & 3) * 32;
       const size_t goff = (static_cast<size_t>(row_base) + wrow0) * p.D + col0;      // in fp32 elements
       const int rows = N - wrow0, cols16 = 2 * (p.D - col0);                          // columns in 16-bit units
-      store_rows_via_smem<2>(patch, q0, reinterpret_cast<uint16_t*>(static_cast<float*>(p.out0) + goff),
+      store_rows_via_smem<2>(patch, q0, reinterpret_cast<uint16_t*>(static_cast<float*>(out0) + goff),
                              2 * static_cast<size_t>(p.D), rows, cols16, lane);
       if constexpr (DUAL)
-        store_rows_via_smem<2>(patch, q1, reinterpret_cast<uint16_t*>(static_cast<float*>(p.out1) + goff),
+        store_rows_via_smem<2>(patch, q1, reinterpret_cast<uint16_t*>(static_cast<float*>(out1) + goff),
                                2 * static_cast<size_t>(p.D), rows, cols16, lane);
     } else {
       constexpr int CH = D / 64;
@@ -839,9 +858,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap rm0, const __grid_constant_
 #pragma unroll
       for (int g = 0; g < C::NACC / 2; ++g) {
         const uint32_t acc = tmem + lane_off + (g == 0 ? C::TMEM_ACC0 : C::TMEM_ACC2);
-        const float scale = (g == 0) ? p.out_scale : 1.0f;
-        void* const o0 = (g == 0) ? p.out0 : p.out2;
-        void* const o1 = (g == 0) ? p.out1 : p.out3;
+        const float scale = (g == 0 && FAM != FAM_V) ? p.s : 1.0f;   // dV, dtV are not scaled
+        void* const o0 = (g == 0) ? out0 : p.dv;
+        void* const o1 = (g == 0) ? out1 : p.dtv;
         uint32_t q0[CH][16], q1[CH][16];
 #pragma unroll
         for (int cc = 0; cc < CH; ++cc) {
@@ -870,6 +889,40 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap rm0, const __grid_constant_
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 9) tmem_dealloc(tmem, C::TMEM_COLS);
+}
+
+// Families of a call in the order of their blocks (longest first), and the shared memory of a launch that holds all of them.
+template <int D, bool SPLIT>
+struct BwdFamilies {
+  static constexpr int COUNT = D == 64 ? 2 : 3;
+  static constexpr int FAM[3] = {D == 64 ? FAM_KV : FAM_K, FAM_Q, FAM_V};
+  static constexpr size_t smem_bytes() {
+    constexpr size_t a = BwdCfg<D, FAM[0], SPLIT>::smem_bytes(), b = BwdCfg<D, FAM_Q, SPLIT>::smem_bytes();
+    constexpr size_t c = COUNT == 3 ? BwdCfg<D, FAM_V, SPLIT>::smem_bytes() : 0;
+    return a > b ? (a > c ? a : c) : (b > c ? b : c);
+  }
+};
+
+// All families in one launch. Every family alone has as many blocks as there are 128-row tiles, which for short sequences
+// or few units leaves most SMs without work or ends in a nearly empty wave, once per launch; together the families fill each
+// other's gaps and cost one launch.
+// The blocks are ordered by family first (the longest family first) and inside a family as in block_work, heavier tiles first
+// under a causal mask (early key tiles, late query tiles). The families' code must not alternate on the SMs: with the families
+// of every group of units next to one another (which would keep the operands in L2) the instruction caches thrash
+// (B=8 H=16 N=4096 D=128 causal 8.4 ms instead of 5.0).
+// Measured against one launch per family (us): B=4 H=8 N=1024 D=128 causal fp16 primal only 102 -> 80; B=32 H=16 N=256 D=72
+// 285 -> 266; B=5 H=7 N=777 D=96 padded 156 -> 126; H=12 N=1024 D=128 94 -> 73; B=4 H=16 N=2048 D=64 694 -> 659; fp32 B=2 H=4
+// N=128 31 -> 12, B=2 H=12 N=2048 692 -> 632; no difference once a family alone has some twenty waves of blocks (B=8 H=16
+// N=4096 D=128 causal).
+template <int D, bool BF16, bool PAD, bool DUAL, bool SPLIT = false, bool DROP = false>
+__global__ void __launch_bounds__(352, 1) bwd_sm100_kernel(const __grid_constant__ BwdMaps maps, const __grid_constant__ BwdKParams p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  using F = BwdFamilies<D, SPLIT>;
+  const int per_fam = p.n_rt * p.n_units, idx = static_cast<int>(blockIdx.x) / per_fam, fam = p.first_fam + idx;
+  const BlockWork work = block_work(static_cast<int>(blockIdx.x) - idx * per_fam, p.n_rt, p.n_units, p.unit_group, p.causal && fam == 1);
+  if (fam == 0) bwd_family<D, F::FAM[0], BF16, PAD, DUAL, SPLIT, DROP>(maps, p, work.tile, work.unit, smem);
+  else if (fam == 1) bwd_family<D, FAM_Q, BF16, PAD, DUAL, SPLIT, DROP>(maps, p, work.tile, work.unit, smem);
+  else if constexpr (F::COUNT == 3) bwd_family<D, FAM_V, BF16, PAD, DUAL, SPLIT, DROP>(maps, p, work.tile, work.unit, smem);
 }
 
 // Where the rows of the upstream gradients start: go and gto may be strided views, o and to are contiguous.
@@ -968,74 +1021,48 @@ __global__ void bwd_preprocess_f32_kernel(const float* __restrict__ o, const flo
   }
 }
 
-// The tensor maps of a backward call, one with the row-side and one with the column-side box per operand: every operand
-// is row-side in one family and column-side in another, so they are encoded once for all launches of the call.
-enum { OP_Q = 0, OP_K, OP_V, OP_GO, OP_TQ, OP_TK, OP_TV, OP_GTO, N_OPS };
-struct BwdMaps {
-  CUtensorMap row[N_OPS], col[N_OPS];
-  bool encode(const jvpfa_bwd_args& a) {
-    const void* const ptr[N_OPS] = {a.q, a.k, a.v, a.go, a.tq, a.tk, a.tv, a.gto};
-    const jvpfa_strides* const st[N_OPS] = {&a.q_strides, &a.k_strides, &a.v_strides, &a.go_strides,
-                                            &a.tq_strides, &a.tk_strides, &a.tv_strides, &a.gto_strides};
-    const bool dual = a.tq != nullptr;
-    for (int i = 0; i < N_OPS; ++i) {
-      if (!dual && i >= OP_TQ) {   // tangent operands of a primal-only call: aliases, never used
-        row[i] = row[i - OP_TQ];
-        col[i] = col[i - OP_TQ];
-        continue;
-      }
-      const TensorView v = make_view(ptr[i], *st[i], a.H, a.N, a.D);
-      if (!make_tile_map(&row[i], v, a.B, a.H, a.N, a.D, 128, a.dtype) || !make_tile_map(&col[i], v, a.B, a.H, a.N, a.D, 64, a.dtype))
-        return false;
-    }
-    return true;
-  }
-};
-
 // `a` holds the operands the tensor maps are built on: in the split-fp32 mode (SPLIT) the bf16 hi/lo tensors of the
 // pre-pass with 128 columns, and `real_D` is the head dimension of the outputs.
-template <int D, int FAM, bool BF16, bool PAD, bool DUAL, bool SPLIT = false, bool DROP = false>
-int launch_family(const jvpfa_bwd_args& a, const BwdMaps& m, const float4* stats, int* status, cudaStream_t stream, int real_D = 0) {
-  using C = BwdCfg<D, FAM, SPLIT>;
-  static_assert(C::BR == 128 && C::BC == 64, "the boxes of BwdMaps");
-  // rows and first / second column pair of the family: query side {q, tq, go, gto} or key side {k, tk, v, tv} (family V
-  // reads k, tk only)
-  const bool rows_q = FAM == FAM_Q;
-  const CUtensorMap* const rm[4] = {&m.row[rows_q ? OP_Q : OP_K], &m.row[rows_q ? OP_TQ : OP_TK], &m.row[rows_q ? OP_GO : OP_V],
-                                    &m.row[rows_q ? OP_GTO : OP_TV]};
-  const CUtensorMap* const cm[4] = {&m.col[rows_q ? OP_K : OP_Q], &m.col[rows_q ? OP_TK : OP_TQ], &m.col[rows_q ? OP_V : OP_GO],
-                                    &m.col[rows_q ? OP_TV : OP_GTO]};
-  void *out0, *out1, *out2 = nullptr, *out3 = nullptr;
-  float out_scale = a.sm_scale;
-  if (FAM == FAM_Q) {
-    out0 = a.dq; out1 = a.dtq;
-  } else if (FAM == FAM_K || FAM == FAM_KV) {
-    out0 = a.dk; out1 = a.dtk;
-    if (FAM == FAM_KV) { out2 = a.dv; out3 = a.dtv; }
-  } else {
-    out0 = a.dv; out1 = a.dtv; out_scale = 1.0f;
-  }
+// With events (`marks`) every family is a launch of its own between two of them, in the order Q, K, V (Q, KV).
+template <int D, bool BF16, bool PAD, bool DUAL, bool SPLIT = false, bool DROP = false>
+int launch_families(const jvpfa_bwd_args& a, const BwdMaps& maps, const float4* stats, int* status, cudaStream_t stream,
+                    const LaunchMarks& marks, int real_D) {
+  using F = BwdFamilies<D, SPLIT>;
   BwdKParams p{};
-  p.H = a.H; p.N = a.N; p.D = SPLIT ? real_D : a.D; p.causal = a.causal;
+  p.H = a.H; p.N = a.N; p.D = real_D; p.causal = a.causal;
   p.s = a.sm_scale;
   p.c1 = a.sm_scale * 1.4426950408889634f;
-  p.out_scale = out_scale;
   p.mv = make_mask_view(a.mask, a.mask_summary, a.B, a.H, a.N);
   p.stats = stats;
-  p.out0 = out0; p.out1 = out1; p.out2 = out2; p.out3 = out3;
+  p.dq = a.dq; p.dtq = a.dtq; p.dk = a.dk; p.dtk = a.dtk; p.dv = a.dv; p.dtv = a.dtv;
   p.status = status;
   p.budget_ns = wait_budget_ns();
   p.drop = make_dropout_params(a.dropout_p, a.dropout_seed);
-  auto kern = bwd_sm100_kernel<D, FAM, BF16, PAD, DUAL, SPLIT, DROP>;
-  const size_t smem = C::smem_bytes();
-  static SmemOptIn opt_in;
-  if (!opt_in.set(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_LAUNCH;
-  p.n_rt = (a.N + C::BR - 1) / C::BR;
+  p.n_rt = (a.N + 127) / 128;
   p.n_units = a.B * a.H;
   p.unit_group = unit_group_size(p.n_units);
-  dim3 grid(static_cast<unsigned>(p.n_rt) * static_cast<unsigned>(p.n_units));
-  kern<<<grid, 352, smem, stream>>>(*rm[0], *rm[1], *rm[2], *rm[3], *cm[0], *cm[1], *cm[2], *cm[3], p);
-  return cudaGetLastError() == cudaSuccess ? JVPFA_OK : JVPFA_ERR_LAUNCH;
+  auto kern = bwd_sm100_kernel<D, BF16, PAD, DUAL, SPLIT, DROP>;
+  const size_t smem = F::smem_bytes();
+  static SmemOptIn opt_in;
+  if (!opt_in.set(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_LAUNCH;
+  auto launch = [&](int first, int n) {
+    p.first_fam = first;
+    kern<<<static_cast<unsigned>(n) * p.n_rt * p.n_units, 352, smem, stream>>>(maps, p);
+    return cudaGetLastError() == cudaSuccess;
+  };
+  marks.mark(1);
+  // (a grid has at most 2^31 - 1 blocks: beyond that, too, one launch per family)
+  if (marks.events == nullptr && static_cast<int64_t>(F::COUNT) * p.n_rt * p.n_units <= 0x7FFFFFFF) {
+    if (!launch(0, F::COUNT)) return JVPFA_ERR_LAUNCH;
+  } else {
+    if (!launch(1, 1)) return JVPFA_ERR_LAUNCH;
+    marks.mark(2);
+    if (!launch(0, 1)) return JVPFA_ERR_LAUNCH;
+    marks.mark(3);
+    if (F::COUNT == 3 && !launch(2, 1)) return JVPFA_ERR_LAUNCH;
+  }
+  marks.mark(4);
+  return JVPFA_OK;
 }
 
 template <bool BF16>
@@ -1059,22 +1086,8 @@ int launch_all(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const 
   BwdMaps maps;
   if (!maps.encode(a)) return JVPFA_ERR_LAUNCH;
   auto three = [&](auto pad, auto dual, auto drop) {
-    constexpr bool P = decltype(pad)::value, DU = decltype(dual)::value, DR = decltype(drop)::value;
-    marks.mark(1);
-    int rc = launch_family<D, FAM_Q, BF16, P, DU, false, DR>(a, maps, stats, status, stream);
-    if (rc != JVPFA_OK) return rc;
-    marks.mark(2);
-    if constexpr (D == 64) {   // the key-side gradients in one pass
-      rc = launch_family<D, FAM_KV, BF16, P, DU, false, DR>(a, maps, stats, status, stream);
-      marks.mark(3);
-    } else {
-      rc = launch_family<D, FAM_K, BF16, P, DU, false, DR>(a, maps, stats, status, stream);
-      if (rc != JVPFA_OK) return rc;
-      marks.mark(3);
-      rc = launch_family<D, FAM_V, BF16, P, DU, false, DR>(a, maps, stats, status, stream);
-    }
-    marks.mark(4);
-    return rc;
+    return launch_families<D, BF16, decltype(pad)::value, decltype(dual)::value, false, decltype(drop)::value>(a, maps, stats, status, stream,
+                                                                                                               marks, a.D);
   };
   const bool dual = a.tq != nullptr;
   if (a.dropout_p > 0.f) {
@@ -1121,16 +1134,7 @@ int launch_split(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, cons
   if (DUAL) { m.tq = dst[4]; m.tk = dst[5]; m.tv = dst[6]; m.gto = dst[7]; }
   BwdMaps maps;
   if (!maps.encode(m)) return JVPFA_ERR_LAUNCH;
-  marks.mark(1);
-  rc = launch_family<128, FAM_Q, true, false, DUAL, true, DROP>(m, maps, stats, status, stream, a.D);
-  if (rc != JVPFA_OK) return rc;
-  marks.mark(2);
-  rc = launch_family<128, FAM_K, true, false, DUAL, true, DROP>(m, maps, stats, status, stream, a.D);
-  if (rc != JVPFA_OK) return rc;
-  marks.mark(3);
-  rc = launch_family<128, FAM_V, true, false, DUAL, true, DROP>(m, maps, stats, status, stream, a.D);
-  marks.mark(4);
-  return rc;
+  return launch_families<128, true, false, DUAL, true, DROP>(m, maps, stats, status, stream, marks, a.D);
 }
 
 }  // namespace
