@@ -931,24 +931,26 @@ struct GradLayout {
   TensorView go, gto;
   __host__ __device__ int64_t offset(int64_t row, const TensorView& v) const {
     if (v.sh == v.sn * N && v.sb == v.sh * H) return row * v.sn;   // rows evenly spaced (the contiguous case)
-    const int64_t n = row % N, bh = row / N;
-    return (bh / H) * v.sb + (bh % H) * v.sh + n * v.sn;
+    const uint32_t r = static_cast<uint32_t>(row), bh = r / N, n = r - bh * N, b = bh / H;   // (a call has below 2^31 rows)
+    return b * v.sb + (bh - b * H) * v.sh + n * v.sn;
   }
 };
 
 // stats[row] = (lse2, mu, Delta, a) with a = rowsum(gtO o O), Delta = rowsum(gO o O) + rowsum(gtO o tO) - a mu.
-// Half a warp per row; 16-bit inputs. Generalises the reference's _attn_bwd_preprocess
-// (jvp_attention.py:1395-1422), which computes rowsum(O o dO) only.
-template <bool BF16>
-__global__ void bwd_preprocess_kernel(const uint16_t* __restrict__ o, const uint16_t* __restrict__ to,
-                                      const uint16_t* __restrict__ go, const uint16_t* __restrict__ gto,
-                                      const float* __restrict__ lse2, const float* __restrict__ mu,
-                                      float4* __restrict__ stats, int64_t rows, int D, const GradLayout gl) {
-  // half a warp per row, 16 bytes per lane and tensor in flight
-  const int lane = threadIdx.x & 31, l16 = lane & 15;
-  const int64_t row = (static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 2 + (lane >> 4);
-  const bool live = row < rows;
-  const int64_t go_row = live ? gl.offset(row, gl.go) : 0, gto_row = live ? gl.offset(row, gl.gto) : 0;
+// Eight lanes per row up to head dimension 64, else half a warp; 16-bit inputs, 16 bytes per lane and tensor. The work is
+// memory latency: a thread has its pieces of ROWS rows in flight. (us, against half a warp per row, one row per thread and
+// 64-bit divisions: B=4 H=16 N=2048 D=64 22 -> 14, primal only 18 -> 10; B=32 H=16 N=256 D=72 transposed gradients 31 -> 23;
+// N=4096 B=8 H=16 D=128 94 -> 93, 5.8 TB/s.)
+// Generalises the reference's _attn_bwd_preprocess (jvp_attention.py:1395-1422), which computes rowsum(O o dO) only.
+constexpr int kPreprocessRows = 2;
+template <bool BF16, int LPR>
+__global__ void __launch_bounds__(256)
+bwd_preprocess_kernel(const uint16_t* __restrict__ o, const uint16_t* __restrict__ to, const uint16_t* __restrict__ go,
+                      const uint16_t* __restrict__ gto, const float* __restrict__ lse2, const float* __restrict__ mu,
+                      float4* __restrict__ stats, int64_t rows, int D, const GradLayout gl) {
+  constexpr int ROWS = kPreprocessRows;
+  const int lane = threadIdx.x & 31, l = lane % LPR;
+  const int64_t row0 = ((static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 / LPR) + lane / LPR) * ROWS;
   auto lo = [](uint32_t x) -> float {
     if constexpr (BF16) return __uint_as_float(x << 16);
     else return __half2float(__ushort_as_half(static_cast<uint16_t>(x & 0xFFFFu)));
@@ -957,34 +959,50 @@ __global__ void bwd_preprocess_kernel(const uint16_t* __restrict__ o, const uint
     if constexpr (BF16) return __uint_as_float(x & 0xFFFF0000u);
     else return __half2float(__ushort_as_half(static_cast<uint16_t>(x >> 16)));
   };
-  float s_go_o = 0.f, s_gto_to = 0.f, s_gto_o = 0.f;
-  if (live) {
-    for (int d = l16 * 8; d < D; d += 128) {
-      const size_t idx = static_cast<size_t>(row) * D + d;
+  int64_t row[ROWS], go_row[ROWS], gto_row[ROWS];
+  float s_go_o[ROWS], s_gto_to[ROWS], s_gto_o[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    row[r] = min(row0 + r, rows - 1);     // (past the end: the last row again, not written)
+    go_row[r] = gl.offset(row[r], gl.go);
+    gto_row[r] = gl.offset(row[r], gl.gto);
+    s_go_o[r] = s_gto_to[r] = s_gto_o[r] = 0.f;
+  }
+  for (int d = l * 8; d < D; d += 8 * LPR) {
+    uint4 v[ROWS][4];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const int64_t idx = row[r] * D + d;
       const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-      const uint4 ov = *reinterpret_cast<const uint4*>(o + idx);
-      const uint4 gov = *reinterpret_cast<const uint4*>(go + go_row + d);
-      const uint4 tov = gto ? *reinterpret_cast<const uint4*>(to + idx) : z;
-      const uint4 gtov = gto ? *reinterpret_cast<const uint4*>(gto + gto_row + d) : z;
-      const uint32_t a0[4] = {ov.x, ov.y, ov.z, ov.w}, a1[4] = {tov.x, tov.y, tov.z, tov.w};
-      const uint32_t a2[4] = {gov.x, gov.y, gov.z, gov.w}, a3[4] = {gtov.x, gtov.y, gtov.z, gtov.w};
+      v[r][0] = *reinterpret_cast<const uint4*>(o + idx);
+      v[r][1] = gto ? *reinterpret_cast<const uint4*>(to + idx) : z;
+      v[r][2] = *reinterpret_cast<const uint4*>(go + go_row[r] + d);
+      v[r][3] = gto ? *reinterpret_cast<const uint4*>(gto + gto_row[r] + d) : z;
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const uint32_t a0[4] = {v[r][0].x, v[r][0].y, v[r][0].z, v[r][0].w}, a1[4] = {v[r][1].x, v[r][1].y, v[r][1].z, v[r][1].w};
+      const uint32_t a2[4] = {v[r][2].x, v[r][2].y, v[r][2].z, v[r][2].w}, a3[4] = {v[r][3].x, v[r][3].y, v[r][3].z, v[r][3].w};
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        s_go_o = fmaf(lo(a2[u]), lo(a0[u]), s_go_o);     s_go_o = fmaf(hi(a2[u]), hi(a0[u]), s_go_o);
-        s_gto_to = fmaf(lo(a3[u]), lo(a1[u]), s_gto_to); s_gto_to = fmaf(hi(a3[u]), hi(a1[u]), s_gto_to);
-        s_gto_o = fmaf(lo(a3[u]), lo(a0[u]), s_gto_o);   s_gto_o = fmaf(hi(a3[u]), hi(a0[u]), s_gto_o);
+        s_go_o[r] = fmaf(lo(a2[u]), lo(a0[u]), s_go_o[r]);     s_go_o[r] = fmaf(hi(a2[u]), hi(a0[u]), s_go_o[r]);
+        s_gto_to[r] = fmaf(lo(a3[u]), lo(a1[u]), s_gto_to[r]); s_gto_to[r] = fmaf(hi(a3[u]), hi(a1[u]), s_gto_to[r]);
+        s_gto_o[r] = fmaf(lo(a3[u]), lo(a0[u]), s_gto_o[r]);   s_gto_o[r] = fmaf(hi(a3[u]), hi(a0[u]), s_gto_o[r]);
       }
     }
   }
 #pragma unroll
-  for (int off = 8; off > 0; off >>= 1) {
-    s_go_o += __shfl_xor_sync(0xFFFFFFFFu, s_go_o, off);
-    s_gto_to += __shfl_xor_sync(0xFFFFFFFFu, s_gto_to, off);
-    s_gto_o += __shfl_xor_sync(0xFFFFFFFFu, s_gto_o, off);
-  }
-  if (l16 == 0 && live) {
-    const float m = mu[row];
-    stats[row] = make_float4(lse2[row], m, s_go_o + s_gto_to - s_gto_o * m, s_gto_o);
+  for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+    for (int off = LPR / 2; off > 0; off >>= 1) {
+      s_go_o[r] += __shfl_xor_sync(0xFFFFFFFFu, s_go_o[r], off);
+      s_gto_to[r] += __shfl_xor_sync(0xFFFFFFFFu, s_gto_to[r], off);
+      s_gto_o[r] += __shfl_xor_sync(0xFFFFFFFFu, s_gto_o[r], off);
+    }
+    if (l == 0 && row0 + r < rows) {
+      const float m = mu[row[r]];
+      stats[row[r]] = make_float4(lse2[row[r]], m, s_go_o[r] + s_gto_to[r] - s_gto_o[r] * m, s_gto_o[r]);
+    }
   }
 }
 
@@ -1068,12 +1086,15 @@ int launch_families(const jvpfa_bwd_args& a, const BwdMaps& maps, const float4* 
 template <bool BF16>
 int launch_preprocess(const jvpfa_bwd_args& a, float4* stats, cudaStream_t stream) {
   const int64_t rows = static_cast<int64_t>(a.B) * a.H * a.N;
-  const int warps_per_block = 8;   // two rows per warp
-  const unsigned blocks = static_cast<unsigned>((rows + 2 * warps_per_block - 1) / (2 * warps_per_block));
   const GradLayout gl{a.H, a.N, make_view(a.go, a.go_strides, a.H, a.N, a.D), make_view(a.gto, a.gto_strides, a.H, a.N, a.D)};
-  bwd_preprocess_kernel<BF16><<<blocks, warps_per_block * 32, 0, stream>>>(
-      static_cast<const uint16_t*>(a.o), static_cast<const uint16_t*>(a.to), static_cast<const uint16_t*>(a.go),
-      static_cast<const uint16_t*>(a.gto), a.lse2, a.mu, stats, rows, a.D, gl);
+  auto go = [&](auto lpr) {
+    constexpr int LPR = decltype(lpr)::value, per_block = 256 / LPR * kPreprocessRows;
+    bwd_preprocess_kernel<BF16, LPR><<<static_cast<unsigned>((rows + per_block - 1) / per_block), 256, 0, stream>>>(
+        static_cast<const uint16_t*>(a.o), static_cast<const uint16_t*>(a.to), static_cast<const uint16_t*>(a.go),
+        static_cast<const uint16_t*>(a.gto), a.lse2, a.mu, stats, rows, a.D, gl);
+  };
+  if (a.D <= 64) go(std::integral_constant<int, 8>{});
+  else go(std::integral_constant<int, 16>{});
   return cudaGetLastError() == cudaSuccess ? JVPFA_OK : JVPFA_ERR_LAUNCH;
 }
 
