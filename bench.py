@@ -461,6 +461,8 @@ def run_cuda(args, rank, world, local_rank):
             acc[nme] += marks[i][j].elapsed_time(marks[i][j + 1])
     kernels = {nme: {"ms_per_launch": acc[nme] / args.steps, "launches": args.steps} for nme in names}
     lfwd_f, lbwd_f = algorithmic_flops(1, U, N, D, causal)            # this rank's slice
+    # main backward launches of a step: one for all families, three from twenty waves of blocks per family on (bwd_sm100.cuh)
+    bwd_launches = 3 if causal and U * ((N + 127) // 128) >= 20 * 148 else 1
     fam_ms = (acc["bwd_q"] + acc["bwd_k"] + acc["bwd_v"]) / (3.0 * args.steps)
     # dominant kernel: the backward kernel, one launch per step; this pass runs its three families as launches of their own,
     # between events; algorithmic FLOPs per
@@ -608,7 +610,7 @@ def run_cuda(args, rank, world, local_rank):
             "frac_of_measured_sustained_peak": value / world / peak_sustained,
             "roofline": roofline, "kernels": kernels, other_name: other_rec, "weak": weak,
             "cpu_baseline": cpu_baseline, "gpu_incumbent": incumbent, "dit": dit, "e2e": e2e,
-            "gpu_launches": 3 * args.steps, "clocks": clocks.summary(),
+            "gpu_launches": (2 + bwd_launches) * args.steps, "clocks": clocks.summary(),
             # time x clock: millions of SM cycles per step at the clock counted beside the kernels (power-cap noise drops out)
             "mcycles_per_step": (ms_step * clocks.in_kernel_mhz / 1e3) if clocks.in_kernel_mhz else None,
         }
