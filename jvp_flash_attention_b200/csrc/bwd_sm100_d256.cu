@@ -67,8 +67,14 @@ __device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams&
   uint64_t* bars = reinterpret_cast<uint64_t*>(ring + kSlots * kSlotBytes + 2 * 4 * 64 * 4);
   uint64_t *full = bars, *empty = bars + kSlots;
   uint64_t &ra_full = bars[2 * kSlots], &rb_full = bars[2 * kSlots + 1], &s_full = bars[2 * kSlots + 2], &s_free = bars[2 * kSlots + 3],
-           &g_full = bars[2 * kSlots + 4], &e_full = bars[2 * kSlots + 5], &acc_final = bars[2 * kSlots + 6];
-  uint64_t* e_free = bars + 2 * kSlots + 7;   // [2]
+           &g_full = bars[2 * kSlots + 4], &acc_final = bars[2 * kSlots + 5];
+  // A barrier must not complete a second phase before its waiter has seen the first. With X, A the element-wise warps meet
+  // the issuer every tile (g_full of tile i + 1 is committed behind outputs(i)), so one e_full does. Without them nothing holds
+  // tile i + 1 back while the issuer is between its commit of S(i + 1) and its wait for e_full of tile i: every buffer of P, tP
+  // has an e_full of its own, and tile i + 2 waits for e_free of outputs(i).
+  constexpr int NE = GR ? 1 : 2;
+  uint64_t* e_full = bars + 2 * kSlots + 6;   // [NE]
+  uint64_t* e_free = bars + 2 * kSlots + 8;   // [2]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = bh / p.H, h = bh % p.H;
@@ -221,7 +227,7 @@ __device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams&
       }
     };
     auto outputs = [&](int i) {
-      wait_all(&e_full, i & 1, 22);
+      wait_all(&e_full[i % NE], (i / NE) & 1, 22);
       // FULL: dS replaces X, dtS replaces A in place (two groups of 16 columns); PV: P, tP in one of two buffers
       const uint32_t EP = T2 + (i & 1) * 64;
       const uint32_t E0 = KIND == KIND_FULL ? (QSIDE ? T2 + 64 : T2) : (KIND == KIND_ONE ? T2 : EP);
@@ -419,7 +425,7 @@ __device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams&
       }
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(&e_full);
+      mbar_arrive(&e_full[it % NE]);
     }
     mbar_wait(&acc_final, 0, w, 33);
     tc_fence_after_sync();
@@ -479,10 +485,11 @@ __global__ void __launch_bounds__(320, 1) bwd_sm100_wide_kernel(const __grid_con
     mbar_init(&bars[2 * kSlots + 2], 1);      // s_full
     mbar_init(&bars[2 * kSlots + 3], 256);    // s_free
     mbar_init(&bars[2 * kSlots + 4], 1);      // g_full
-    mbar_init(&bars[2 * kSlots + 5], 256);    // e_full
-    mbar_init(&bars[2 * kSlots + 6], 1);      // acc_final
-    mbar_init(&bars[2 * kSlots + 7], 1);      // e_free
-    mbar_init(&bars[2 * kSlots + 8], 1);
+    mbar_init(&bars[2 * kSlots + 5], 1);      // acc_final
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars[2 * kSlots + 6 + i], 256);   // e_full
+      mbar_init(&bars[2 * kSlots + 8 + i], 1);     // e_free
+    }
     fence_mbar_init();
   }
   __syncthreads();

@@ -44,3 +44,31 @@ def test_wide_heads(dev, dtype, D, N, kind):
         assert float((t.double().cpu() - torch.from_numpy(ref[n])).abs().max()) <= 2e-2, n
     torch.cuda.synchronize()
     _lib.read_status(dev)
+
+
+@pytest.mark.parametrize("dtype,B,H,N,D,causal,dual", [
+    (torch.bfloat16, 2, 40, 257, 256, True, True), (torch.float16, 3, 25, 130, 136, False, True),
+    (torch.bfloat16, 2, 2, 2500, 192, False, True), (torch.float16, 2, 2, 2500, 256, False, False),
+])
+def test_many_units_equal_few(dev, dtype, B, H, N, D, causal, dual):
+    """A backward with more blocks than SMs, or with 40 column tiles a block (the value families then run through their score
+    buffers many times), against the same (batch, head) units in calls of their own: the same bits."""
+    from jvp_flash_attention_b200 import _lib
+    g = torch.Generator(device=dev).manual_seed(N + D)
+    ts = [torch.randn(B, H, N, D, device=dev, generator=g).to(dtype) for _ in range(8)]
+
+    def run(b, h):
+        q, k, v, tq, tk, tv, go, gto = (t[b, h].contiguous() for t in ts)
+        if not dual:
+            tq = tk = tv = gto = None
+        mask = _lib.make_mask(None, *q.shape[:3])
+        o, to, lse2, mu = _lib.fwd(q, k, v, tq, tk, tv, mask, None, causal, D ** -0.5)
+        return _lib.bwd(q, k, v, tq, tk, tv, o, to, lse2, mu, go, gto, mask, None, causal, D ** -0.5)
+
+    whole = run(slice(None), slice(None))
+    assert all(t.isfinite().all() for t in whole)
+    for h in (0, H // 2, H - 1):
+        part = run(slice(B - 1, B), slice(h, h + 1))
+        assert all(torch.equal(a[B - 1, h], b[0, 0]) for a, b in zip(whole, part)), h
+    torch.cuda.synchronize()
+    _lib.read_status(dev)
