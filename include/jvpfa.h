@@ -47,7 +47,7 @@ typedef struct jvpfa_mask {
 
 /* Element strides of a (B,H,N,D) input tensor along B, H and N; the D axis must be contiguous. All zero means the
  * contiguous layout (H*N*D, N*D, D). A strided input (for instance q = qkv.permute(2,0,3,1,4)[0] of a fused projection,
- * or an upstream gradient that is a transposed view) is read in place by the tensor-core kernels when every stride
+ * or an upstream gradient that is a transposed view) is read in place by the tensor-core paths when every stride
  * is a multiple of 16 bytes and the pointer is 16-byte aligned; otherwise, and for the shapes that run on the
  * CUDA-core kernels (head dimension above 256 or not a multiple of 8; fp32 above 64), the call returns
  * JVPFA_ERR_UNSUPPORTED and the caller copies the tensor first. */
@@ -118,8 +118,10 @@ const char* jvpfa_error_string(int status);
 /* Bytes of caller-provided scratch the calls below want (always >= 256: the first 4 bytes hold the device status
  * word that bounded waits write to; it must be zero before the first call). For fp32 inputs with a head dimension
  * of at most 64 this is the need of the tensor-core path, which keeps bf16 hi/lo splits of its operands in the
- * workspace (256 bytes per row and tensor); a call that is given less, but at least 256 bytes (forward) or
- * 256 + 16 bytes per row (backward), runs the same mathematics on the CUDA cores instead. */
+ * workspace (256 bytes per row and tensor); for fp16 inputs with a head dimension of 136 to 256 likewise (4 bytes per element
+ * of v, tv in the forward, of q, k, go and their tangents in the backward, for as many batches at a time as fit 1 GiB, or one).
+ * A call that is given less, but at least 256 bytes (forward) or 256 + 16 bytes per row (backward), runs the same mathematics
+ * on the CUDA cores instead (contiguous inputs only). Everything else needs exactly that much. */
 size_t jvpfa_fwd_workspace_bytes(const jvpfa_fwd_args* args);
 size_t jvpfa_bwd_workspace_bytes(const jvpfa_bwd_args* args);
 
@@ -194,7 +196,8 @@ int jvpfa_selftest_timeout(void* workspace, int32_t budget_us, int32_t* out4, vo
  * make that first call before starting any stream capture. With CUDA's default lazy module loading that
  * look-up is also where the driver sets the array up on the device, so a process whose memory pool is about
  * to claim the rest of the GPU's memory makes the first call before the pool grows (or sets
- * CUDA_MODULE_LOADING=EAGER). fp32 inputs run on the CUDA-core kernels here. Every call clears the status word at the
+ * CUDA_MODULE_LOADING=EAGER). fp32 inputs, and fp16 ones with a head dimension
+ * above 128, run on the CUDA-core kernels here. Every call clears the status word at the
  * start of the array on `stream` and then reuses the rest as it is. All calls on a device share the
  * one array: two calls whose kernels can overlap on the GPU (different streams without an ordering
  * between them) race on it and give undefined results -- order them yourself.

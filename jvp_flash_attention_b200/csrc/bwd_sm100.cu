@@ -12,6 +12,13 @@ size_t bwd_sm100_workspace_bytes(const jvpfa_bwd_args& a) {
   return kStatusBytes + static_cast<size_t>(a.B) * a.H * a.N * sizeof(float4);
 }
 
+// bf16: what every path takes. fp16: the split operands of the output products behind it.
+size_t bwd_sm100_wide_workspace_bytes(const jvpfa_bwd_args& a) {
+  const size_t stats = static_cast<size_t>(a.B) * a.H * a.N * sizeof(float4);
+  return a.dtype == JVPFA_F16 ? kStatusBytes + align_up(stats, 256) + split_f16_bytes(a.tq != nullptr ? 6 : 3, a.B, a.H, a.N, a.D)
+                              : kStatusBytes + stats;
+}
+
 int launch_bwd_sm100(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const LaunchMarks& marks) {
   const bool bf = a.dtype == JVPFA_BF16;
   if (a.D > 128) return launch_bwd_sm100_d256(a, status, stream, marks);

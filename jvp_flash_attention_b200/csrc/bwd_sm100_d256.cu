@@ -8,10 +8,17 @@
 //   * the operands that S, tS are made of stay resident (128 KB), everything else streams through a ring of six 16 KB slots
 //     in 64-column slabs: a slab of a stacked column pair [c0; c1], a slab of a row-side operand of X and A, and the
 //     column slabs once more for the output products.
+//   * probabilities and score gradients keep 16 bits of significand and the range of fp32: they go to TMEM as bf16 hi and lo parts,
+//     which take the place of the 32-bit score tile they come from, and meet bf16 columns c as e_hi c + e_lo c. fp16 columns come
+//     split into bf16 hi + lo (exact; a product cannot take an fp16 operand against a bf16 one; a pre-pass writes them to the
+//     workspace): e_hi c_hi + e_lo c_hi + e_hi c_lo. Rounded to the inputs' 16 bits instead, the gradients' errors were 1.3 to 1.5
+//     times those of the fp32 CUDA-core kernels, and fp16 score gradients above 65504 overflowed.
 // One launch holds the blocks of all families, heaviest family first: a launch per family leaves most of the SMs idle
 // behind the longest row tile of a causal problem when there are few (batch, head) units.
-// B=2 H=8 N=1024 D=256 causal fp16: 0.232 ms (12.2 ms on the CUDA cores).
-// Bound: the slab stream (320 KB per 128 x 64 tile of dQ or dK at 256 columns, against 4.3 k cycles of MMA).
+// Whole call, us, B=2 H=8 N=1024 D=256 causal: bf16 268, fp16 325 with its pre-pass (16-bit probabilities and score gradients: 282,
+// 286; CUDA cores, fp16: 12364); B=4 H=8 N=2048 causal: 1615, 2026 (1480, 1494); B=16 H=16 N=256: 579, 749 (586, 583).
+// Bound: the slab stream (320 KB per 128 x 64 tile of dQ or dK at 256 columns, fp16 384 KB) and the output products (twice, fp16
+// three times, those of 16-bit operands).
 //
 // Warps 0-7 element-wise (two warpgroups that split the 64 columns of a tile), warp 8 TMA producer, warp 9 MMA issuer; one
 // static order of slots per block that producer and issuer both walk:
@@ -22,6 +29,7 @@ namespace jvpfa {
 namespace {
 
 enum { KIND_FULL = 0, KIND_ONE = 1, KIND_PV2 = 2, KIND_PV1 = 3 };
+// (the columns c of the output products are operands out[] of the maps)
 //   FULL: S, tS, X, A -> out = dS c0 + dtS c1          (dQ, dK)
 //   ONE:  S, Y        -> out = E c0, E = P (Y - stat)  (dtQ, dtK with Y = A, stat a; primal-only dQ, dK with Y = X, stat Delta)
 //   PV2:  S, tS       -> out = P c2 + tP c3            (dV)
@@ -36,8 +44,14 @@ struct WideFamily {
 };
 constexpr int kMaxFamilies = 6;
 
+struct WideMaps {
+  BwdMaps in;
+  CUtensorMap out[N_OPS];   // columns of the output products: bf16 inputs as they are, fp16 inputs split (hi at column 0, lo at D)
+};
+
 struct WideParams {
   int H, N, D;
+  int b0;                   // first batch of this launch; fp16: where the out maps begin
   int n_rt, n_units, unit_group, n_fam;
   int causal;
   float c1, s;
@@ -56,10 +70,12 @@ constexpr int kWideBars = 2 * kSlots + 10;
 constexpr size_t kWideSmem = 2 * kRowTile + kSlots * kSlotBytes + 2 * 4 * 64 * 4 + (kWideBars + 2) * 8;
 
 template <int KIND, bool QSIDE, bool BF16>
-__device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams& p, const WideFamily& f, int rt, int bh, uint8_t* smem,
+__device__ __forceinline__ void wide_body(const WideMaps& wm, const WideParams& p, const WideFamily& f, int rt, int bh, uint8_t* smem,
                                           uint32_t tmem, const WaitCtx& w) {
   constexpr bool TS = KIND == KIND_FULL || KIND == KIND_PV2;     // tangent scores
   constexpr bool GR = KIND == KIND_FULL || KIND == KIND_ONE;     // score products of the upstream gradients
+  constexpr int PARTS = BF16 ? 1 : 2;                            // column slabs of an output product: c, or c_hi and c_lo
+  const BwdMaps& maps = wm.in;
   uint8_t* const sRA = smem;
   uint8_t* const sRB = smem + kRowTile;
   uint8_t* const ring = smem + 2 * kRowTile;
@@ -69,12 +85,12 @@ __device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams&
   uint64_t &ra_full = bars[2 * kSlots], &rb_full = bars[2 * kSlots + 1], &s_full = bars[2 * kSlots + 2], &s_free = bars[2 * kSlots + 3],
            &g_full = bars[2 * kSlots + 4], &acc_final = bars[2 * kSlots + 5];
   // A barrier must not complete a second phase before its waiter has seen the first. With X, A the element-wise warps meet
-  // the issuer every tile (g_full of tile i + 1 is committed behind outputs(i)), so one e_full does. Without them nothing holds
-  // tile i + 1 back while the issuer is between its commit of S(i + 1) and its wait for e_full of tile i: every buffer of P, tP
-  // has an e_full of its own, and tile i + 2 waits for e_free of outputs(i).
-  constexpr int NE = GR ? 1 : 2;
+  // the issuer every tile (g_full of tile i + 1 is committed behind outputs(i)), with P, tP in one buffer they wait for e_free of
+  // outputs(i), so one e_full does. With two buffers nothing holds tile i + 1 back while the issuer is between its commit of
+  // S(i + 1) and its wait for e_full of tile i: every buffer has an e_full of its own, and tile i + 2 waits for e_free of outputs(i).
+  constexpr int NE = KIND == KIND_PV1 ? 2 : 1;   // 64 columns of P hi, lo; P, tP hi, lo take all 128
   uint64_t* e_full = bars + 2 * kSlots + 6;   // [NE]
-  uint64_t* e_free = bars + 2 * kSlots + 8;   // [2]
+  uint64_t* e_free = bars + 2 * kSlots + 8;   // [NE]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = bh / p.H, h = bh % p.H;
@@ -137,9 +153,17 @@ __device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams&
         }
       };
       auto outputs = [&](int j) {
+        const CUtensorMap *m0 = &wm.out[GR ? f.c[0] : f.c[2]], *m1 = &wm.out[GR ? f.c[1] : f.c[3]];
         for (int sl = 0; sl < n_slabs; ++sl) {
-          if constexpr (GR) slot_cols(f.c[0], KIND == KIND_FULL ? f.c[1] : -1, sl, j * 64);
-          else slot_cols(f.c[2], KIND == KIND_PV2 ? f.c[3] : -1, sl, j * 64);
+#pragma unroll
+          for (int part = 0; part < PARTS; ++part) {
+            const int x = part * D + 64 * sl, bo = BF16 ? b : b - p.b0;
+            mbar_wait(&empty[slot], phase ^ 1, w, 12);
+            mbar_arrive_expect_tx(&full[slot], TS ? kSlotBytes : kHalfSlot);
+            tma_load_tile(ring + slot * kSlotBytes, m0, &full[slot], x, j * 64, h, bo);
+            if constexpr (TS) tma_load_tile(ring + slot * kSlotBytes + kHalfSlot, m1, &full[slot], x, j * 64, h, bo);
+            advance();
+          }
         }
       };
       load_rows(sRA, f.r[0], &ra_full);
@@ -169,7 +193,7 @@ __device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams&
     };
     constexpr uint32_t FMT = BF16 ? FMT_BF16 : FMT_F16;
     const uint32_t idesc_64 = make_idesc(FMT, 128, 64, 0, 0), idesc_128 = make_idesc(FMT, 128, 128, 0, 0);
-    const uint32_t idesc_out = make_idesc(FMT, 128, 64, 0, 1);
+    const uint32_t idesc_out = make_idesc(FMT_BF16, 128, 64, 0, 1);
     const uint32_t T0 = tmem + 256, T2 = T0 + 128;
     const int ksteps = (D + 15) / 16;
     auto wait_slot = [&]() {
@@ -228,26 +252,33 @@ __device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams&
     };
     auto outputs = [&](int i) {
       wait_all(&e_full[i % NE], (i / NE) & 1, 22);
-      // FULL: dS replaces X, dtS replaces A in place (two groups of 16 columns); PV: P, tP in one of two buffers
-      const uint32_t EP = T2 + (i & 1) * 64;
-      const uint32_t E0 = KIND == KIND_FULL ? (QSIDE ? T2 + 64 : T2) : (KIND == KIND_ONE ? T2 : EP);
-      const uint32_t E1 = KIND == KIND_FULL ? (QSIDE ? T2 : T2 + 64) : EP + 32;
+      // FULL: dS replaces X, dtS replaces A in place, PV: P, tP beside the scores; of 64 score columns, each warpgroup's 32 become
+      // 16 columns of hi and 16 of lo parts
+      const uint32_t E0 = KIND == KIND_FULL ? (QSIDE ? T2 + 64 : T2) : (GR ? T2 : T2 + (i % NE) * 64);
+      const uint32_t E1 = KIND == KIND_FULL && QSIDE ? T2 : T2 + 64;
       for (int sl = 0; sl < n_slabs; ++sl) {
-        wait_slot();
-        const uint64_t d0 = desc_mnmajor_sw128(smem_u32(ring + slot * kSlotBytes), kSlotBytes);
-        const uint64_t d1 = desc_mnmajor_sw128(smem_u32(ring + slot * kSlotBytes + kHalfSlot), kSlotBytes);
         const uint32_t acc = tmem + 64 * sl;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t ek = GR ? (k & 1) * 8 + (k >> 1) * 32 : k * 8;
-          const uint64_t dk = static_cast<uint64_t>((k * 2048) >> 4);
-          umma_ts_pred(acc, E0 + ek, d0 + dk, idesc_out, i > 0 || k > 0, lead);
-          if constexpr (TS) umma_ts_pred(acc, E1 + ek, d1 + dk, idesc_out, 1, lead);
+        for (int part = 0; part < PARTS; ++part) {
+          wait_slot();
+          const uint64_t d0 = desc_mnmajor_sw128(smem_u32(ring + slot * kSlotBytes), kSlotBytes);
+          const uint64_t d1 = desc_mnmajor_sw128(smem_u32(ring + slot * kSlotBytes + kHalfSlot), kSlotBytes);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint32_t hi = (k & 1) * 8 + (k >> 1) * 32, lo = hi + 16;
+            const uint64_t dk = static_cast<uint64_t>((k * 2048) >> 4);
+            umma_ts_pred(acc, E0 + hi, d0 + dk, idesc_out, i > 0 || part > 0 || k > 0, lead);
+            if (part == 0) umma_ts_pred(acc, E0 + lo, d0 + dk, idesc_out, 1, lead);
+            if constexpr (TS) {
+              umma_ts_pred(acc, E1 + hi, d1 + dk, idesc_out, 1, lead);
+              if (part == 0) umma_ts_pred(acc, E1 + lo, d1 + dk, idesc_out, 1, lead);
+            }
+          }
+          release(&empty[slot]);
+          advance();
         }
-        release(&empty[slot]);
-        advance();
       }
-      if constexpr (!GR) release(&e_free[i & 1]);
+      if constexpr (!GR) release(&e_free[i % NE]);
     };
     wait_all(&ra_full, 0, 23);
     if constexpr (KIND != KIND_PV1) wait_all(&rb_full, 0, 24);
@@ -283,6 +314,21 @@ __device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams&
       if (st.x == -INFINITY) nst.x = -INFINITY;   // fully excluded query: P = 0
     }
     const float2 c1_2 = make_float2(p.c1, p.c1), s_2 = make_float2(p.s, p.s);
+    // this thread's 32 values of a tile, pair i = value(i), as 16 columns of hi and 16 of lo parts from TMEM column `col` on
+    auto store_hi_lo = [](uint32_t col, auto value) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint32_t hi[8], lo[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float2 v = value(8 * q + i);
+          hi[i] = pack2<true>(v.x, v.y);
+          lo[i] = pack2_residual(v.x, v.y, hi[i]);
+        }
+        tmem_st_x8(col + 8 * q, hi);
+        tmem_st_x8(col + 16 + 8 * q, lo);
+      }
+    };
     auto fetch_stats = [&](int j) -> float4 {   // statistics of the next column tile, fetched one tile ahead
       float4 sv = make_float4(INFINITY, 0.f, 0.f, 0.f);
       if (!QSIDE && tid < 64 && j < j_end && j * 64 + tid < N) sv = __ldg(&p.stats[row_base + j * 64 + tid]);
@@ -367,61 +413,35 @@ __device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams&
         tc_fence_after_sync();
         const uint32_t TY = T0 + 128 + 32 * wg;                                   // KIND_ONE
         const uint32_t TA = QSIDE ? TY : TY + 64, TX = QSIDE ? TY + 64 : TY;      // KIND_FULL
-        if constexpr (KIND == KIND_FULL) {
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {   // A -> dtS = P (A - a), and everything of dS that does not need X
-            uint32_t ar[16], e[8];
-            tmem_ld_x16(TA + 16 * q, ar);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int ip = 8 * q + i;
-              const float2 A = make_float2(__uint_as_float(ar[2 * i]), __uint_as_float(ar[2 * i + 1]));
-              const float2 d = __fadd2_rn(A, stat2(3, ip));
-              const float2 t = __ffma2_rn(ts2[ip], d, stat2(2, ip));              // ts (A - a) - Delta
-              ts2[ip] = __ffma2_rn(stat2(1, ip), A, t);                           // - mu A
-              const float2 v = __fmul2_rn(P2[ip], d);
-              e[i] = pack2<BF16>(v.x, v.y);
-            }
-            tmem_st_x8(TA + 8 * q, e);
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {     // X -> dS = P (X + the above), or Y -> E = P (Y - stat)
-          uint32_t xr[16], e[8];
-          tmem_ld_x16((KIND == KIND_FULL ? TX : TY) + 16 * q, xr);
+        if constexpr (KIND == KIND_FULL) {   // A -> dtS = P (A - a), and everything of dS that does not need X
+          uint32_t ar[32];
+          tmem_ld_x32(TA, ar);
           tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int ip = 8 * q + i;
-            const float2 X = make_float2(__uint_as_float(xr[2 * i]), __uint_as_float(xr[2 * i + 1]));
-            const float2 add = KIND == KIND_FULL ? ts2[ip] : (f.stat == 2 ? stat2(2, ip) : stat2(3, ip));
-            const float2 v = __fmul2_rn(P2[ip], __fadd2_rn(X, add));
-            e[i] = pack2<BF16>(v.x, v.y);
-          }
-          tmem_st_x8((KIND == KIND_FULL ? TX : TY) + 8 * q, e);
+          store_hi_lo(TA, [&](int i) -> float2 {
+            const float2 A = make_float2(__uint_as_float(ar[2 * i]), __uint_as_float(ar[2 * i + 1]));
+            const float2 d = __fadd2_rn(A, stat2(3, i));
+            const float2 t = __ffma2_rn(ts2[i], d, stat2(2, i));                // ts (A - a) - Delta
+            ts2[i] = __ffma2_rn(stat2(1, i), A, t);                             // - mu A
+            return __fmul2_rn(P2[i], d);
+          });
         }
+        // X -> dS = P (X + the above), or Y -> E = P (Y - stat)
+        uint32_t xr[32];
+        tmem_ld_x32(KIND == KIND_FULL ? TX : TY, xr);
+        tmem_wait_ld();
+        store_hi_lo(KIND == KIND_FULL ? TX : TY, [&](int i) -> float2 {
+          const float2 X = make_float2(__uint_as_float(xr[2 * i]), __uint_as_float(xr[2 * i + 1]));
+          const float2 add = KIND == KIND_FULL ? ts2[i] : (f.stat == 2 ? stat2(2, i) : stat2(3, i));
+          return __fmul2_rn(P2[i], __fadd2_rn(X, add));
+        });
       } else {
-        const uint32_t EP = T0 + 128 + (it & 1) * 64 + 16 * wg;   // this thread's 16 columns of P; tP is 32 columns further
-        if (it >= 2) {   // the output products of tile it - 2 read this buffer
-          mbar_wait(&e_free[it & 1], ((it >> 1) - 1) & 1, w, 32);
+        const uint32_t EP = T0 + 128 + (it % NE) * 64 + 32 * wg;   // this thread's columns of P hi, lo; tP is 64 columns further
+        if (it >= NE) {   // the output products of tile it - NE read this buffer
+          mbar_wait(&e_free[it % NE], (it / NE - 1) & 1, w, 32);
           tc_fence_after_sync();
         }
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          uint32_t e0[8], e1[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int ip = 8 * q + i;
-            e0[i] = pack2<BF16>(P2[ip].x, P2[ip].y);
-            if constexpr (TS) {
-              const float2 tp = __fmul2_rn(P2[ip], __fadd2_rn(ts2[ip], stat2(1, ip)));
-              e1[i] = pack2<BF16>(tp.x, tp.y);
-            }
-          }
-          tmem_st_x8(EP + 8 * q, e0);
-          if constexpr (TS) tmem_st_x8(EP + 32 + 8 * q, e1);
-        }
+        store_hi_lo(EP, [&](int i) -> float2 { return P2[i]; });
+        if constexpr (TS) store_hi_lo(EP + 64, [&](int i) -> float2 { return __fmul2_rn(P2[i], __fadd2_rn(ts2[i], stat2(1, i))); });
       }
       tmem_wait_st();
       tc_fence_before_sync();
@@ -461,7 +481,7 @@ __device__ __forceinline__ void wide_body(const BwdMaps& maps, const WideParams&
 }
 
 template <bool BF16>
-__global__ void __launch_bounds__(320, 1) bwd_sm100_wide_kernel(const __grid_constant__ BwdMaps maps, const __grid_constant__ WideParams p) {
+__global__ void __launch_bounds__(320, 1) bwd_sm100_wide_kernel(const __grid_constant__ WideMaps maps, const __grid_constant__ WideParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * kRowTile + kSlots * kSlotBytes + 2 * 4 * 64 * 4);
   uint32_t& tmem_base_s = *reinterpret_cast<uint32_t*>(bars + kWideBars);
@@ -477,7 +497,7 @@ __global__ void __launch_bounds__(320, 1) bwd_sm100_wide_kernel(const __grid_con
   const int per_fam = p.n_rt * p.n_units, fi = static_cast<int>(blockIdx.x) / per_fam;
   const WideFamily& f = p.fam[fi];
   const BlockWork work = block_work(static_cast<int>(blockIdx.x) - fi * per_fam, p.n_rt, p.n_units, p.unit_group, p.causal && f.qside);
-  const int rt = work.tile;
+  const int rt = work.tile, bh = work.unit + p.b0 * p.H;
   const WaitCtx w{p.status, &poisoned, p.budget_ns};
   if (threadIdx.x == 0) {
     poisoned = 0;
@@ -502,15 +522,15 @@ __global__ void __launch_bounds__(320, 1) bwd_sm100_wide_kernel(const __grid_con
   tc_fence_after_sync();
   const uint32_t tmem = warp == 8 ? 0u : tmem_base_s;
   if (f.kind == KIND_FULL) {
-    if (f.qside) wide_body<KIND_FULL, true, BF16>(maps, p, f, rt, work.unit, smem, tmem, w);
-    else wide_body<KIND_FULL, false, BF16>(maps, p, f, rt, work.unit, smem, tmem, w);
+    if (f.qside) wide_body<KIND_FULL, true, BF16>(maps, p, f, rt, bh, smem, tmem, w);
+    else wide_body<KIND_FULL, false, BF16>(maps, p, f, rt, bh, smem, tmem, w);
   } else if (f.kind == KIND_ONE) {
-    if (f.qside) wide_body<KIND_ONE, true, BF16>(maps, p, f, rt, work.unit, smem, tmem, w);
-    else wide_body<KIND_ONE, false, BF16>(maps, p, f, rt, work.unit, smem, tmem, w);
+    if (f.qside) wide_body<KIND_ONE, true, BF16>(maps, p, f, rt, bh, smem, tmem, w);
+    else wide_body<KIND_ONE, false, BF16>(maps, p, f, rt, bh, smem, tmem, w);
   } else if (f.kind == KIND_PV2) {
-    wide_body<KIND_PV2, false, BF16>(maps, p, f, rt, work.unit, smem, tmem, w);
+    wide_body<KIND_PV2, false, BF16>(maps, p, f, rt, bh, smem, tmem, w);
   } else {
-    wide_body<KIND_PV1, false, BF16>(maps, p, f, rt, work.unit, smem, tmem, w);
+    wide_body<KIND_PV1, false, BF16>(maps, p, f, rt, bh, smem, tmem, w);
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -524,8 +544,8 @@ int launch_wide(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const
   marks.mark(0);
   const int rc = launch_preprocess<BF16>(a, stats, stream);
   if (rc != JVPFA_OK) return rc;
-  BwdMaps maps;
-  if (!maps.encode(a)) return JVPFA_ERR_LAUNCH;
+  WideMaps maps;
+  if (!maps.in.encode(a)) return JVPFA_ERR_LAUNCH;
   WideParams p{};
   p.H = a.H; p.N = a.N; p.D = a.D; p.causal = a.causal;
   p.s = a.sm_scale;
@@ -562,19 +582,43 @@ int launch_wide(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const
     add(KIND_PV1, false, a.dv, 1.f, 0, false);
   }
   p.n_rt = (a.N + 127) / 128;
-  p.n_units = a.B * a.H;
   // All row tiles of a group of units come before the next group's, so the group bounds both the tail (heaviest blocks first
   // only inside a group) and the tensors that the running blocks stream: eight per unit, kept to half of L2.
   const size_t unit_bytes = 16 * static_cast<size_t>(a.N) * a.D;
   const int fit = static_cast<int>((size_t{64} << 20) / unit_bytes);
-  p.unit_group = fit < 1 ? 1 : (fit < p.n_units ? fit : p.n_units);
   auto kern = bwd_sm100_wide_kernel<BF16>;
   static SmemOptIn opt_in;
   if (!opt_in.set(reinterpret_cast<const void*>(kern), kWideSmem)) return JVPFA_ERR_LAUNCH;
   marks.mark(1);
-  kern<<<static_cast<unsigned>(p.n_fam) * p.n_rt * p.n_units, 320, kWideSmem, stream>>>(maps, p);
+  // the columns of the output products; fp16: a launch per group of batches whose split tensors fit the workspace
+  const int n_out = dual ? 6 : 3, ops[6] = {OP_Q, OP_K, OP_GO, OP_TQ, OP_TK, OP_GTO};
+  const int step = BF16 ? a.B : split_f16_batches(n_out, a.B, a.H, a.N, a.D);
+  const void* const src[6] = {a.q, a.k, a.go, a.tq, a.tk, a.gto};
+  const jvpfa_strides* const st[6] = {&a.q_strides, &a.k_strides, &a.go_strides, &a.tq_strides, &a.tk_strides, &a.gto_strides};
+  uint16_t* const split = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(stats) +
+                                                      align_up(static_cast<size_t>(a.B) * a.H * a.N * sizeof(float4), 256));
+  for (int b0 = 0; b0 < a.B; b0 += step) {
+    const int nb = a.B - b0 < step ? a.B - b0 : step;
+    for (int i = 0; i < N_OPS; ++i) maps.out[i] = maps.in.col[i];
+    if constexpr (!BF16) {
+      TensorView views[6];
+      uint16_t* dst[6];
+      for (int i = 0; i < n_out; ++i) {
+        views[i] = batches_from(make_view(src[i], *st[i], a.H, a.N, a.D), b0, 2);
+        dst[i] = split + i * split_f16_elems(step, a.H, a.N, a.D);
+        if (!make_split_f16_map(&maps.out[ops[i]], dst[i], nb, a.H, a.N, a.D, 64)) return JVPFA_ERR_LAUNCH;
+      }
+      const int rc_split = launch_split_f16(views, dst, n_out, nb, a.H, a.N, a.D, stream);
+      if (rc_split != JVPFA_OK) return rc_split;
+    }
+    p.b0 = b0;
+    p.n_units = nb * a.H;
+    p.unit_group = fit < 1 ? 1 : (fit < p.n_units ? fit : p.n_units);
+    kern<<<static_cast<unsigned>(p.n_fam) * p.n_rt * p.n_units, 320, kWideSmem, stream>>>(maps, p);
+    if (cudaGetLastError() != cudaSuccess) return JVPFA_ERR_LAUNCH;
+  }
   for (int i = 2; i < 5; ++i) marks.mark(i);
-  return cudaGetLastError() == cudaSuccess ? JVPFA_OK : JVPFA_ERR_LAUNCH;
+  return JVPFA_OK;
 }
 
 }  // namespace

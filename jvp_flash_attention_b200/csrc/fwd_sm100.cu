@@ -21,6 +21,10 @@ size_t fwd_sm100_split_workspace_bytes(const jvpfa_fwd_args& a) {
   return kStatusBytes + (a.tq != nullptr ? 6 : 3) * rows * kSplitRowBytes;
 }
 
+size_t fwd_sm100_wide_workspace_bytes(const jvpfa_fwd_args& a) {
+  return kStatusBytes + (a.dtype == JVPFA_F16 ? split_f16_bytes(a.tq != nullptr ? 2 : 1, a.B, a.H, a.N, a.D) : 0);
+}
+
 int launch_fwd_sm100(const jvpfa_fwd_args& a, int* status, cudaStream_t stream) {
   if (a.D <= 64) return launch_fwd_sm100_d64(a, status, stream);
   return a.D <= 128 ? launch_fwd_sm100_d128(a, status, stream) : launch_fwd_sm100_d256(a, status, stream);

@@ -43,6 +43,7 @@ struct FwdKParams {
   float c1;      // sm_scale * log2(e)
   float s;       // sm_scale
   float thresh;  // lazy-rescale threshold in the log2 domain
+  int b0;        // D = 256: first batch of this launch (fp16: where the tensor maps of the split V, tV begin)
   MaskView mv;
   void* o;
   void* to;
@@ -85,12 +86,14 @@ struct FwdCfg {
   static constexpr int BM = 128;
   static constexpr int BN = 64;
   static constexpr bool WIDE = D > 128;           // half of the output columns per CTA, see the kernel
-  static constexpr int STAGES = (D == 64) ? 4 : (WIDE ? 1 : 2);   // V, tV tiles
+  static constexpr bool HILO = SPLIT || WIDE;     // P and W as bf16 hi and lo parts
+  static constexpr int STAGES = (D == 64) ? 4 : 2;                // slots of V, tV tiles (WIDE: of one tile of either)
   static constexpr int KSB = WIDE ? 1 : D / 64;   // 64-column slabs of [K; tK] per barrier
   static constexpr int KST = WIDE ? D / 64 : STAGES;              // ring slots of KSB slabs
   static constexpr int DV = SPLIT ? 64 : (WIDE ? D / 2 : D);      // columns of the O and T accumulators
   static constexpr int TILE_Q = BM * D * 2;
   static constexpr int TILE_V = BN * (WIDE ? DV : D) * 2;
+  static constexpr int SLOT_V = WIDE ? TILE_V : 2 * TILE_V;
   static constexpr int SLAB = 128 * 128;          // bytes of one 64-column slab of a 128-row tile
   static constexpr int SLOT_K = KSB * SLAB;       // K and tK stacked as one 128-row operand
   static constexpr int HALF = BN * 128;           // byte offset of tK inside a slab of the pair
@@ -98,11 +101,12 @@ struct FwdCfg {
   static constexpr int TMEM_T = DV;
   static constexpr int TMEM_S = 2 * DV;       // S 64 columns, tS 64 columns further (one buffer)
   static constexpr int TMEM_P = 2 * DV + 128; // 16-bit P (32 columns) and W (32 columns further), buffer b at + PBUF b;
-  static constexpr int PBUF = SPLIT ? 128 : 64;  // SPLIT: P hi, P lo, W hi, W lo, 32 columns each
+  static constexpr int PBUF = HILO ? 128 : 64;   // HILO: P hi, P lo, W hi, W lo, 32 columns each
+  static constexpr int PBUFS = WIDE ? 1 : 2;
   static constexpr int TMEM_COLS = 512;
   static constexpr int NBAR = 4 + 2 * KST + 2 * STAGES + 4 + 2;
   static constexpr size_t smem_bytes() {
-    return 2 * TILE_Q + KST * SLOT_K + STAGES * 2 * TILE_V + 2 * 2 * 128 * 4 + (NBAR + 2) * 8;
+    return 2 * TILE_Q + KST * SLOT_K + STAGES * SLOT_V + 2 * 2 * 128 * 4 + (NBAR + 2) * 8;
   }
 };
 
@@ -112,8 +116,15 @@ struct FwdCfg {
 // TMEM allocation.
 // D = 256 (head dimensions 136 to 256): O and T alone would fill TMEM, so two CTAs share a query tile, each with half of
 // the output columns (V, tV columns) and all of the score products: 9 tile products where one CTA would run 6. Q, tQ take
-// 128 KB of shared memory; K, tK go through four 16 KB slots by 64-column slab, V, tV have one 32 KB buffer.
-// B=2 H=8 N=1024 D=256 causal fp16: 0.063 ms (3.11 ms on the CUDA cores).
+// 128 KB of shared memory; K, tK go through four 16 KB slots by 64-column slab, V, tV through two of one tile.
+// P and W keep 16 bits of significand and the range of fp32: they go to TMEM as bf16 hi and lo parts (one buffer, where the
+// narrower kernels have two of 16-bit numbers). bf16 inputs: P V = P_hi V + P_lo V. fp16 inputs: a product cannot take an fp16
+// operand against a bf16 one, so V, tV come split into bf16 hi and lo (exact, a pre-pass writes them to the workspace) and P V =
+// P_hi V_hi + P_lo V_hi + P_hi V_lo. With P and W rounded to the inputs' 16 bits the outputs' errors were 1.24 to 1.5 times those
+// of the fp32 CUDA-core kernels.
+// B=2 H=8 N=1024 D=256 causal, us: bf16 72, fp16 108 with its pre-pass (16-bit P and W: 76, 77; CUDA cores, fp16: 3314); B=4 H=8
+// N=2048: 330, 482 (292, 285). Errors against 64 bits over those of the CUDA cores (D = 136, 192, 256, N = 64 to 1024): bf16 1.000,
+// fp16 1.000 to 1.001; 1.010 at N = 4096 (the tensor cores' fp32 accumulation).
 // PAD: the tensors' head dimension is smaller than D (columns beyond it are zero-filled by TMA); the K steps and
 // output columns that would only see zeros are then skipped at run time.
 // DROP: dropout on the attention probabilities (dropout.cuh): P and W reach TMEM dropped out and rescaled, the row sums l
@@ -128,16 +139,17 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   constexpr int ST = C::STAGES, KST = C::KST;
   constexpr int SLABS = D / 64;
   constexpr int DV = C::DV;
-  constexpr int VSLABS = C::WIDE ? DV / 64 : SLABS;   // slabs of a V tile
+  constexpr int VSLABS = DV / 64;                     // WIDE: slabs of a V tile,
+  constexpr int VD = DUAL ? 2 : 1, VT = BF16 ? VD : 2 * VD;   // tiles of V, tV (fp16: their hi parts, then the lo parts) per key tile
   static_assert(!SPLIT || (D == 128 && BF16 && !PAD), "the split-fp32 mode runs on the 128-column geometry in bf16");
 
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem;
   uint8_t* sTQ = sQ + C::TILE_Q;
   auto sK = [&](int slot) { return smem + 2 * C::TILE_Q + slot * C::SLOT_K; };   // slabs of the [K; tK] pair
-  auto sV = [&](int st) { return smem + 2 * C::TILE_Q + KST * C::SLOT_K + st * 2 * C::TILE_V; };
+  auto sV = [&](int st) { return smem + 2 * C::TILE_Q + KST * C::SLOT_K + st * C::SLOT_V; };
   auto sTV = [&](int st) { return sV(st) + C::TILE_V; };
-  uint8_t* tail = smem + 2 * C::TILE_Q + KST * C::SLOT_K + ST * 2 * C::TILE_V;
+  uint8_t* tail = smem + 2 * C::TILE_Q + KST * C::SLOT_K + ST * C::SLOT_V;
   float(*xch)[2][128] = reinterpret_cast<float(*)[2][128]>(tail);          // [parity][warpgroup][row]
   uint64_t* bars = reinterpret_cast<uint64_t*>(tail + 2 * 2 * 128 * 4);
   uint64_t& q_full = bars[0];
@@ -166,7 +178,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int dcol0 = half * dcols;
   const int n_slabs = C::WIDE && PAD ? (p.D + 63) / 64 : SLABS;           // slabs of K, tK that hold data
   const int qt = work.tile;
-  const int bh = work.unit;
+  const int bh = C::WIDE ? work.unit + p.b0 * p.H : work.unit;
   const int b = bh / p.H, h = bh % p.H;
   const int q0 = qt * C::BM;
   const int N = p.N;
@@ -224,20 +236,33 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       int it = 0;
       for (int j = 0; j < n_kt; ++j) {
         if (!(tile_bits(j) & kTileAnyKept)) continue;
+        const int krow = j * C::BN;   // first key row of the tile inside its (batch, head) unit
+        if constexpr (C::WIDE) {      // V, tV, and with fp16 inputs their lo parts: a slot each
+#pragma unroll
+          for (int n = 0; n < VT; ++n, ++it) {
+            const int st = it % ST, x = (n / VD) * p.D + dcol0;
+            const CUtensorMap* tm = DUAL && n % VD == 1 ? &tmTV : &tmV;
+            mbar_wait(&v_empty[st], ((it / ST) & 1) ^ 1, w, 11);
+            mbar_arrive_expect_tx(&v_full[st], C::TILE_V);
+#pragma unroll
+            for (int sl = 0; sl < VSLABS; ++sl)
+              tma_load_tile(sV(st) + sl * C::HALF, tm, &v_full[st], x + 64 * sl, krow, h, BF16 ? b : b - p.b0);
+          }
+          continue;
+        }
         const int st = it % ST;
         const uint32_t ph = (it / ST) & 1;
-        const int krow = j * C::BN;   // first key row of the tile inside its (batch, head) unit
         mbar_wait(&v_empty[st], ph ^ 1, w, 11);
         mbar_arrive_expect_tx(&v_full[st], (DUAL ? 2 : 1) * C::TILE_V);
-        if constexpr (!PAD && !C::WIDE && SLABS > 1) {
+        if constexpr (!PAD && SLABS > 1) {
           // the slabs of a V tile are consecutive in shared memory: one box per tensor through the 3-D map
           tma_load_slabs(sV(st), &tmV, &v_full[st], krow, h, b);
           if constexpr (DUAL) tma_load_slabs(sTV(st), &tmTV, &v_full[st], krow, h, b);
         } else {
 #pragma unroll
-          for (int sl = 0; sl < VSLABS; ++sl) {
-            tma_load_tile(sV(st) + sl * C::HALF, &tmV, &v_full[st], dcol0 + 64 * sl, krow, h, b);
-            if constexpr (DUAL) tma_load_tile(sTV(st) + sl * C::HALF, &tmTV, &v_full[st], dcol0 + 64 * sl, krow, h, b);
+          for (int sl = 0; sl < SLABS; ++sl) {
+            tma_load_tile(sV(st) + sl * C::HALF, &tmV, &v_full[st], 64 * sl, krow, h, b);
+            if constexpr (DUAL) tma_load_tile(sTV(st) + sl * C::HALF, &tmTV, &v_full[st], 64 * sl, krow, h, b);
           }
         }
         ++it;
@@ -291,7 +316,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t idesc_128 = make_idesc(FMT, 128, 128, 0, 0);
     const int dn = SPLIT ? 64 : (C::WIDE ? dcols : (PAD ? ((p.D + 15) & ~15) : D));   // columns of the output products (rounded up to the MMA granularity)
     const int ksteps = C::WIDE ? (p.D + 15) / 16 : dn / 16;   // K steps of the score products that hold data
-    const uint32_t idesc_pv = make_idesc(FMT, 128, dn, 0, 1);
+    const uint32_t idesc_pv = make_idesc(C::HILO ? FMT_BF16 : FMT, 128, dn, 0, 1);
     const uint64_t dQ = desc_kmajor_sw128(smem_u32(sQ)), dTQ = desc_kmajor_sw128(smem_u32(sTQ));
 
     auto issue_qk = [&](int it) {
@@ -368,9 +393,44 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     auto issue_pv = [&](int it, bool last) {
       const int st = it % ST;
       const uint32_t ph = (it / ST) & 1;
-      const uint32_t P_t = tmem + C::TMEM_P + (it & 1) * C::PBUF;
-      const uint32_t W_t = P_t + (SPLIT ? 64 : 32);
-      wait_all(&p_full[it & 1], (it >> 1) & 1, 21);
+      const uint32_t P_t = tmem + C::TMEM_P + (it % C::PBUFS) * C::PBUF;
+      const uint32_t W_t = P_t + (C::HILO ? 64 : 32);
+      wait_all(&p_full[it % C::PBUFS], (it / C::PBUFS) & 1, 21);
+      if constexpr (C::WIDE) {
+#pragma unroll
+        for (int n = 0; n < VT; ++n) {
+          const int c = it * VT + n, slot = c % ST;
+          wait_all(&v_full[slot], (c / ST) & 1, 22);
+          tc_fence_after_sync();
+          if (leader) {
+            const uint64_t dV = desc_mnmajor_sw128(smem_u32(sV(slot)), C::BN * 128);
+            const bool lo = n >= VD;       // the lo part of V, tV: multiplies the hi parts of P, W only
+            // acc += e_hi c (+ e_lo c)
+            auto mul = [&](uint32_t accum, uint32_t e, uint64_t d, uint32_t first_acc) {
+              umma_ts(accum, e, d, idesc_pv, first_acc);
+              if (!lo) umma_ts(accum, e + 32, d, idesc_pv, 1);
+            };
+#pragma unroll
+            for (int k = 0; k < C::BN / 16; ++k) {
+              const uint64_t d = dV + static_cast<uint64_t>((k * 2048) >> 4);
+              const uint32_t acc = it > 0 || n > 0 || k > 0;
+              if (n % VD == 0) {
+                mul(tmem + C::TMEM_O, P_t + 8 * k, d, acc);
+                if constexpr (DUAL) mul(tmem + C::TMEM_T, W_t + 8 * k, d, acc);
+              } else {
+                mul(tmem + C::TMEM_T, P_t + 8 * k, d, 1);
+              }
+            }
+            umma_commit(&v_empty[slot]);
+            if (n == VT - 1) {
+              umma_commit(&p_free[0]);
+              umma_commit(&o_done);
+              if (last) umma_commit(&o_final);
+            }
+          }
+        }
+        return;
+      }
       wait_all(&v_full[st], ph, 22);
       tc_fence_after_sync();
       const uint64_t dV0 = desc_mnmajor_sw128(smem_u32(sV(st)), C::BN * 128);
@@ -444,8 +504,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (!(bits & kTileAnyKept)) continue;
       const uint32_t S_t = tmem + C::TMEM_S + lane_off + 32 * wg;
       const uint32_t tS_t = S_t + 64;
-      const uint32_t P_t = tmem + C::TMEM_P + (it & 1) * C::PBUF + lane_off + 16 * wg;   // this thread's 16 columns of P
-      const uint32_t W_t = P_t + (SPLIT ? 64 : 32);
+      const uint32_t P_t = tmem + C::TMEM_P + (it % C::PBUFS) * C::PBUF + lane_off + 16 * wg;   // this thread's 16 columns of P
+      const uint32_t W_t = P_t + (C::HILO ? 64 : 32);
       mbar_wait(&s_full, it & 1, w, 30);
       tc_fence_after_sync();
       // scores of this thread's 32 columns in the log2 domain, two per register pair (packed fp32x2
@@ -537,9 +597,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       uint32_t keep_bits = 0xFFFFFFFFu;
       if constexpr (DROP) keep_bits = dropout_keep_along_k(p.drop, bh, qi, k0);
       {
-        // the PV products of tile it - 2 read this P, W buffer
-        if (it >= 2) {
-          mbar_wait(&p_free[it & 1], ((it >> 1) - 1) & 1, w, 33);
+        // the PV products of tile it - PBUFS read this P, W buffer
+        if (it >= C::PBUFS) {
+          mbar_wait(&p_free[it % C::PBUFS], (it / C::PBUFS - 1) & 1, w, 33);
           tc_fence_after_sync();
         }
 #pragma unroll
@@ -554,28 +614,28 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             float2 keep2 = make_float2(1.f, 1.f);
             if constexpr (DROP) keep2 = dropout_factors(keep_bits, ip, p.drop.inv_keep);
             const float2 pd = DROP ? __fmul2_rn(pp, keep2) : pp;     // what multiplies V, tV
-            pk[i] = pack2<BF16>(pd.x, pd.y);
-            if constexpr (SPLIT) pkl[i] = pack2_residual(pd.x, pd.y, pk[i]);
+            pk[i] = pack2<BF16 || C::HILO>(pd.x, pd.y);
+            if constexpr (C::HILO) pkl[i] = pack2_residual(pd.x, pd.y, pk[i]);
             if constexpr (DUAL) {
               const float2 tsv = __fmul2_rn(make_float2(__uint_as_float(ts[2 * ip]), __uint_as_float(ts[2 * ip + 1])), s_2);
               const float2 ww = __fmul2_rn(pp, tsv);
               mu2 = __fadd2_rn(mu2, ww);
               const float2 wd = DROP ? __fmul2_rn(ww, keep2) : ww;
-              wk[i] = pack2<BF16>(wd.x, wd.y);
-              if constexpr (SPLIT) wkl[i] = pack2_residual(wd.x, wd.y, wk[i]);
+              wk[i] = pack2<BF16 || C::HILO>(wd.x, wd.y);
+              if constexpr (C::HILO) wkl[i] = pack2_residual(wd.x, wd.y, wk[i]);
             }
           }
           tmem_st_x8(P_t + 8 * c, pk);
-          if constexpr (SPLIT) tmem_st_x8(P_t + 32 + 8 * c, pkl);
+          if constexpr (C::HILO) tmem_st_x8(P_t + 32 + 8 * c, pkl);
           if constexpr (DUAL) {
             tmem_st_x8(W_t + 8 * c, wk);
-            if constexpr (SPLIT) tmem_st_x8(W_t + 32 + 8 * c, wkl);
+            if constexpr (C::HILO) tmem_st_x8(W_t + 32 + 8 * c, wkl);
           }
         }
       }
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(&p_full[it & 1]);
+      mbar_arrive(&p_full[it % C::PBUFS]);
       ++it;
     }
     // epilogue: total row sums over both warpgroups, then each warpgroup writes half of the head dimension.
@@ -700,18 +760,43 @@ int launch_one(const jvpfa_fwd_args& a, int* status, cudaStream_t stream) {
     return (!PAD && D == 128) ? make_slab_map(m, make_view(ptr, st, a.H, a.N, a.D), a.B, a.H, a.N, a.D, C::BN, a.dtype)
                             : tile(m, ptr, st, C::BN);
   };
-  bool ok = tile(&mQ, a.q, a.q_strides, C::BM) && tile(&mK, a.k, a.k_strides, C::BN) && vmap(&mV, a.v, a.v_strides);
+  constexpr bool SPLIT_V = C::WIDE && !BF16;   // V, tV are read as bf16 hi and lo parts
+  bool ok = tile(&mQ, a.q, a.q_strides, C::BM) && tile(&mK, a.k, a.k_strides, C::BN) && (SPLIT_V || vmap(&mV, a.v, a.v_strides));
   if (DUAL) {
-    ok = ok && tile(&mTQ, a.tq, a.tq_strides, C::BM) && tile(&mTK, a.tk, a.tk_strides, C::BN) && vmap(&mTV, a.tv, a.tv_strides);
+    ok = ok && tile(&mTQ, a.tq, a.tq_strides, C::BM) && tile(&mTK, a.tk, a.tk_strides, C::BN) && (SPLIT_V || vmap(&mTV, a.tv, a.tv_strides));
   } else {
     mTQ = mQ; mTK = mK; mTV = mV;
   }
   if (!ok) return JVPFA_ERR_LAUNCH;
-  const FwdKParams p = make_fwd_params<BF16>(a, status);
+  FwdKParams p = make_fwd_params<BF16>(a, status);
   auto kern = fwd_sm100_kernel<D, DUAL, BF16, PAD, false, DROP>;
   const size_t smem = C::smem_bytes();
   static SmemOptIn opt_in;
   if (!opt_in.set(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_LAUNCH;
+  if constexpr (SPLIT_V) {
+    // a launch per group of batches whose split tensors fit the workspace
+    const void* src[2] = {a.v, a.tv};
+    const jvpfa_strides* st[2] = {&a.v_strides, &a.tv_strides};
+    uint16_t* dst[2];
+    const int n_t = DUAL ? 2 : 1, step = split_f16_batches(n_t, a.B, a.H, a.N, a.D);
+    for (int i = 0; i < n_t; ++i)
+      dst[i] = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(a.workspace) + kStatusBytes) + i * split_f16_elems(step, a.H, a.N, a.D);
+    for (int b0 = 0; b0 < a.B; b0 += step) {
+      const int nb = a.B - b0 < step ? a.B - b0 : step;
+      TensorView views[2];
+      for (int i = 0; i < n_t; ++i) views[i] = batches_from(make_view(src[i], *st[i], a.H, a.N, a.D), b0, 2);
+      const int rc = launch_split_f16(views, dst, n_t, nb, a.H, a.N, a.D, stream);
+      if (rc != JVPFA_OK) return rc;
+      if (!make_split_f16_map(&mV, dst[0], nb, a.H, a.N, a.D, C::BN) || !make_split_f16_map(&mTV, dst[n_t - 1], nb, a.H, a.N, a.D, C::BN))
+        return JVPFA_ERR_LAUNCH;
+      p.b0 = b0;
+      p.n_units = nb * a.H;
+      p.unit_group = unit_group_size(p.n_units);
+      kern<<<static_cast<unsigned>(p.n_qt) * static_cast<unsigned>(p.n_units) * 2u, 384, smem, stream>>>(mQ, mTQ, mK, mTK, mV, mTV, p);
+      if (cudaGetLastError() != cudaSuccess) return JVPFA_ERR_LAUNCH;
+    }
+    return JVPFA_OK;
+  }
   dim3 grid(static_cast<unsigned>(p.n_qt) * static_cast<unsigned>(p.n_units) * (C::WIDE ? 2u : 1u));
   kern<<<grid, 384, smem, stream>>>(mQ, mTQ, mK, mTK, mV, mTV, p);
   return cudaGetLastError() == cudaSuccess ? JVPFA_OK : JVPFA_ERR_LAUNCH;

@@ -91,6 +91,28 @@ struct LaunchMarks {
 constexpr int kSplitMaxTensors = 8;
 constexpr size_t kSplitRowBytes = 256;   // one split row: 64 hi + 64 lo bf16 numbers
 int launch_split_fp32(const TensorView* src, uint16_t* const* dst, int n_tensors, int B, int H, int N, int D, cudaStream_t stream);
+
+// fp16 inputs with a head dimension above 128: the operands that meet probabilities or score gradients are split into bf16 hi + lo
+// parts (11 bits of significand in 8 + 8: exact, with the range of fp32), contiguous rows [hi(D) | lo(D)], for at most
+// kSplitF16Bytes of the workspace at a time (or one batch).
+constexpr size_t kSplitF16Bytes = size_t{1} << 30;
+inline size_t split_f16_elems(int B, int H, int N, int D) { return align_up(static_cast<size_t>(B) * H * N * 2 * D, 128); }   // 256 bytes
+inline int split_f16_batches(int n_tensors, int B, int H, int N, int D) {
+  const size_t fit = kSplitF16Bytes / (2 * n_tensors * split_f16_elems(1, H, N, D));
+  return fit < 1 ? 1 : (fit < static_cast<size_t>(B) ? static_cast<int>(fit) : B);
+}
+inline size_t split_f16_bytes(int n_tensors, int B, int H, int N, int D) {
+  return 2 * n_tensors * split_f16_elems(split_f16_batches(n_tensors, B, H, N, D), H, N, D);
+}
+inline TensorView batches_from(const TensorView& v, int b0, int elem_bytes) {
+  return TensorView{static_cast<const uint8_t*>(v.ptr) + static_cast<int64_t>(b0) * v.sb * elem_bytes, v.sb, v.sh, v.sn};
+}
+inline bool make_split_f16_map(CUtensorMap* out, const uint16_t* split, int B, int H, int N, int D, int box_rows) {
+  return make_tile_map(out, make_view(split, jvpfa_strides{0, 0, 0}, H, N, 2 * D), B, H, N, 2 * D, box_rows, JVPFA_BF16);
+}
+int launch_split_f16(const TensorView* src, uint16_t* const* dst, int n_tensors, int B, int H, int N, int D, cudaStream_t stream);
+size_t fwd_sm100_wide_workspace_bytes(const jvpfa_fwd_args& a);
+size_t bwd_sm100_wide_workspace_bytes(const jvpfa_bwd_args& a);
 bool sm100_split_path_supported(int dtype, int D, int N);
 size_t fwd_sm100_split_workspace_bytes(const jvpfa_fwd_args& a);
 size_t bwd_sm100_split_workspace_bytes(const jvpfa_bwd_args& a);

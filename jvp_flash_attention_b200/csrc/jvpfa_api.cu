@@ -534,6 +534,7 @@ const char* jvpfa_error_string(int status) {
 
 size_t jvpfa_fwd_workspace_bytes(const jvpfa_fwd_args* a) {
   if (a != nullptr && sm100_split_path_supported(a->dtype, a->D, a->N)) return fwd_sm100_split_workspace_bytes(*a);
+  if (a != nullptr && sm100_wide_path_supported(a->dtype, a->D, a->N)) return fwd_sm100_wide_workspace_bytes(*a);
   return kStatusBytes;
 }
 
@@ -541,6 +542,7 @@ size_t jvpfa_bwd_workspace_bytes(const jvpfa_bwd_args* a) {
   if (a == nullptr) return kStatusBytes;
   if (sm100_path_supported(a->dtype, a->D, a->N)) return bwd_sm100_workspace_bytes(*a);
   if (sm100_split_path_supported(a->dtype, a->D, a->N)) return bwd_sm100_split_workspace_bytes(*a);
+  if (sm100_wide_path_supported(a->dtype, a->D, a->N)) return bwd_sm100_wide_workspace_bytes(*a);
   return bwd_generic_workspace_bytes(*a);
 }
 
@@ -648,8 +650,11 @@ int jvpfa_fwd_status(const jvpfa_fwd_args* a, int32_t* status, void* stream) {
       !(sm100_split_path_supported(a->dtype, a->D, a->N) && a->workspace_bytes >= fwd_sm100_split_workspace_bytes(*a)))
     return JVPFA_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (sm100_path_supported(a->dtype, a->D, a->N) || sm100_wide_path_supported(a->dtype, a->D, a->N)) return launch_fwd_sm100(*a, status, s);
-  // fp32: the tensor-core path when the workspace has room for the split operands, else the CUDA-core kernels
+  if (sm100_path_supported(a->dtype, a->D, a->N)) return launch_fwd_sm100(*a, status, s);
+  // fp32, and fp16 above head dimension 128: the tensor-core path when the workspace has room for the split operands, else the
+  // CUDA-core kernels
+  if (sm100_wide_path_supported(a->dtype, a->D, a->N) && a->workspace_bytes >= fwd_sm100_wide_workspace_bytes(*a))
+    return launch_fwd_sm100(*a, status, s);
   if (sm100_split_path_supported(a->dtype, a->D, a->N) && a->workspace_bytes >= fwd_sm100_split_workspace_bytes(*a))
     return launch_fwd_sm100_split(*a, status, s);
   {
@@ -701,8 +706,11 @@ int bwd_checked(const jvpfa_bwd_args* a, int* status, void* stream, void* const*
   LaunchMarks marks;
   marks.events = events;
   marks.stream = s;
-  if (sm100_path_supported(eff.dtype, eff.D, eff.N) || sm100_wide_path_supported(eff.dtype, eff.D, eff.N)) return launch_bwd_sm100(eff, status, s, marks);
-  // fp32: the tensor-core path when the workspace has room for the split operands, else the CUDA-core kernels
+  if (sm100_path_supported(eff.dtype, eff.D, eff.N)) return launch_bwd_sm100(eff, status, s, marks);
+  // fp32, and fp16 above head dimension 128: the tensor-core path when the workspace has room for the split operands, else the
+  // CUDA-core kernels
+  if (sm100_wide_path_supported(eff.dtype, eff.D, eff.N) && eff.workspace_bytes >= bwd_sm100_wide_workspace_bytes(eff))
+    return launch_bwd_sm100(eff, status, s, marks);
   if (sm100_split_path_supported(eff.dtype, eff.D, eff.N) && eff.workspace_bytes >= bwd_sm100_split_workspace_bytes(eff))
     return launch_bwd_sm100_split(eff, status, s, marks);
   {

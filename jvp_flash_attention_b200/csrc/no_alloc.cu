@@ -62,8 +62,8 @@ extern "C" int jvpfa_bwd_noalloc(const jvpfa_bwd_args* args, int32_t* status_wor
   if (cudaMemsetAsync(scratch, 0, jvpfa::kStatusBytes, s) != cudaSuccess) return JVPFA_ERR_LAUNCH;
   jvpfa_bwd_args with_scratch = *args;
   with_scratch.workspace = scratch;
-  // exactly what the status word and the statistics take: fp32 inputs therefore run on the CUDA-core kernels here
-  // (their tensor-core path would want room for split operands that this fixed array does not have)
+  // exactly what the status word and the statistics take: fp32 inputs, and fp16 above head dimension 128, run on the CUDA cores here
+  // (their tensor-core paths would want room for split operands that this fixed array does not have)
   with_scratch.workspace_bytes = jvpfa::kStatusBytes + static_cast<size_t>(rows) * 16;
   rc = jvpfa_bwd(&with_scratch, stream);
   if (rc != JVPFA_OK) return rc;
