@@ -18,6 +18,7 @@
 #include <torch/csrc/utils/pybind.h>
 #include <torch/library.h>
 #include <torch/torch.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cmath>
 #include <mutex>
@@ -355,13 +356,22 @@ std::vector<Tensor> fwd_autograd(const Tensor& q, const Tensor& k, const Tensor&
   return out;
 }
 
-std::vector<Tensor> bwd_autograd(const OptTensor& go, const OptTensor& gto, const Tensor& q, const Tensor& k, const Tensor& v,
+std::vector<Tensor> bwd_autograd(const OptTensor& go_, const OptTensor& gto_, const Tensor& q, const Tensor& k, const Tensor& v,
                                  const OptTensor& tq, const OptTensor& tk, const OptTensor& tv, const Tensor& o, const OptTensor& to,
                                  const Tensor& stats, const OptTensor& mask, const OptTensor& summary, bool causal, double scale,
                                  double dropout_p, int64_t dropout_seed) {
-  if (has_fw_grad(go) || has_fw_grad(gto) || has_fw_grad(q) || has_fw_grad(k) || has_fw_grad(v) || has_fw_grad(tq) ||
-      has_fw_grad(tk) || has_fw_grad(tv))
+  if (has_fw_grad(q) || has_fw_grad(k) || has_fw_grad(v) || has_fw_grad(tq) || has_fw_grad(tk) || has_fw_grad(tv))
     TORCH_CHECK_NOT_IMPLEMENTED(false, kNoNesting);
+  // A backward inside fwAD.dual_level(): whatever nonlinear follows the attention gives upstream gradients that carry a tangent,
+  // from the activations it saved. The gradients are those of the upstream gradients without it. Under torch.func.jvp the
+  // tangent is what the caller asks for: refused (a functorch level is being worked on).
+  const auto without_tangent = [](const OptTensor& t) -> OptTensor {
+    if (!has_fw_grad(t)) return t;
+    if (c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerBackMode))
+      TORCH_CHECK_NOT_IMPLEMENTED(false, kNoNesting);
+    return t->_fw_primal(/*level=*/0);
+  };
+  const OptTensor go = without_tangent(go_), gto = without_tangent(gto_);
   std::vector<Tensor> out;
   {
     at::AutoDispatchBelowADInplaceOrView guard;

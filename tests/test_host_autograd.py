@@ -1,0 +1,116 @@
+"""The autograd side of the native host path on the CPU: its operators with stand-ins for the kernels (the mathematics in plain
+torch), so that what is recorded, saved and refused around the kernels is looked at without a GPU."""
+from concurrent.futures import ThreadPoolExecutor
+
+import pytest
+import torch
+import torch.autograd.forward_ad as fwAD
+import torch.nn.functional as F
+
+B, H, N, D = 2, 2, 6, 8
+
+
+def _scores(q, k, tq, tk, mask, causal, scale):
+    s = q @ k.transpose(-1, -2) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(s.shape[-2:], dtype=torch.bool).triu(1), float("-inf"))
+    if mask is not None:
+        s = s.masked_fill(~mask, float("-inf"))
+    ts = None if tq is None else (tq @ k.transpose(-1, -2) + q @ tk.transpose(-1, -2)) * scale
+    return s.softmax(-1), ts
+
+
+def _outputs(q, k, v, tq, tk, tv, mask, causal, scale):
+    p, ts = _scores(q, k, tq, tk, mask, causal, scale)
+    if tq is None:
+        return [p @ v]
+    w = p * (ts - (p * ts).sum(-1, keepdim=True))
+    return [p @ v, w @ v + p @ tv]
+
+
+def _fwd(q, k, v, tq, tk, tv, mask, causal, scale, dropout_p, seed, verify, tangents_taken):
+    out = _outputs(q, k, v, tq, tk, tv, mask, causal, scale)
+    out.append(torch.zeros(2, *q.shape[:3]))
+    if mask is not None:
+        out.append(torch.zeros(64, dtype=torch.uint8))
+    return out
+
+
+def _bwd(go, gto, q, k, v, tq, tk, tv, o, to, stats, mask, summary, causal, scale, dropout_p, seed):
+    def gradients():
+        ins = [t.detach().requires_grad_() for t in ((q, k, v) if gto is None else (q, k, v, tq, tk, tv))]
+        outs = _outputs(*ins, *([None] * (6 - len(ins))), mask, causal, scale)
+        ups = [torch.zeros_like(q) if go is None else go.detach(), None if gto is None else gto.detach()]
+        return list(torch.autograd.grad(outs, ins, ups[:len(outs)]))
+
+    with ThreadPoolExecutor(1) as thread:      # (a thread of its own: here, below autograd, nothing is recorded)
+        return thread.submit(gradients).result()
+
+
+@pytest.fixture(scope="module")
+def ops(built_library):
+    from jvp_flash_attention_b200 import _lib
+    _lib.host()
+    lib = torch.library.Library("jvpfa", "IMPL")
+    # (below autograd: the kernels see plain tensors)
+    lib.impl("fwd", lambda *a: [t.detach() for t in _fwd(*a)], "CPU")
+    lib.impl("bwd", _bwd, "CPU")
+    yield torch.ops.jvpfa
+    lib._destroy()
+
+
+def _call(ops, q, k, v, mask=None):
+    return ops.attention(q, k, v, mask, False, D ** -0.5, 0.0, 0, False, True)
+
+
+def _dual(ops, *ts, mask=None):
+    return ops.attention_dual(*ts, mask, False, D ** -0.5, 0.0, 0, False)
+
+
+def _inputs(n=6, requires_grad=True):
+    g = torch.Generator().manual_seed(0)
+    return [torch.randn(B, H, N, D, generator=g).requires_grad_(requires_grad) for _ in range(n)]
+
+
+def _layer(ops, x, w):
+    q, k, v = (F.layer_norm(x, (D,)) @ w[i] for i in range(3))
+    y = x + _call(ops, q, k, v)
+    return y + F.gelu(F.layer_norm(y, (D,)) @ w[3])
+
+
+@pytest.mark.parametrize("tangent_of", ["input", "weights too"])
+def test_backward_inside_the_dual_level(ops, tangent_of):
+    """Nonlinear layers behind the attention hand it an upstream gradient that carries a tangent while the level is open: the
+    gradients are those of a backward after the level, and of the same model without the operator."""
+    x, t, gy = _inputs(3, requires_grad=False)
+    g = torch.Generator().manual_seed(1)
+    w = [(torch.randn(D, D, generator=g) / 3).requires_grad_() for _ in range(4)]
+    tw = [torch.randn(D, D, generator=g) / 3 for _ in range(4)]
+
+    def grads(inside, call_ops):
+        with fwAD.dual_level():
+            ws = [fwAD.make_dual(a, b) for a, b in zip(w, tw)] if tangent_of == "weights too" else w
+            y, ty = fwAD.unpack_dual(_layer(call_ops, fwAD.make_dual(x, t), ws))
+            loss = (y * gy).sum() + ty.square().sum()
+            if inside:
+                return torch.autograd.grad(loss, w)
+        return torch.autograd.grad(loss, w)
+
+    class Plain:
+        @staticmethod
+        def attention(q, k, v, mask, causal, scale, *_):
+            (q, tq), (k, tk), (v, tv) = (fwAD.unpack_dual(a) for a in (q, k, v))
+            return fwAD.make_dual(*_outputs(q, k, v, tq, tk, tv, mask, causal, scale))
+
+    want = grads(False, Plain)
+    for inside in (False, True):
+        for a, b in zip(grads(inside, ops), want):
+            torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-5)
+
+
+def test_tangent_of_an_upstream_gradient_is_not_dropped_silently(ops):
+    """Under ``torch.func.jvp`` the tangent of the result is asked for: differentiating the backward raises."""
+    q, k, v, go, tgo = _inputs(5, requires_grad=False)
+    pull = lambda g: torch.func.vjp(lambda a: _call(ops, a, k, v), q)[1](g)[0]
+    with pytest.raises(RuntimeError, match="not supported"):
+        torch.func.jvp(pull, (go,), (tgo,))
