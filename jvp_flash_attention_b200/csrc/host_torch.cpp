@@ -337,7 +337,8 @@ std::vector<Tensor> fwd_autograd(const Tensor& q, const Tensor& k, const Tensor&
   std::shared_ptr<AttentionBackward> node(new AttentionBackward(), torch::autograd::deleteNode);
   if (dual) node->set_next_edges(torch::autograd::collect_next_edges(q, k, v, *tq, *tk, *tv));
   else node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
-  const auto plain = [&](const Tensor& t) { return SavedVariable(tangents_taken && has_fw_grad(t) ? t.detach() : t, false); };
+  // (without the tangent but with its place in the graph, which is what tells bwd_autograd that the gradients depend on it)
+  const auto plain = [&](const Tensor& t) { return SavedVariable(tangents_taken && has_fw_grad(t) ? t._fw_primal(/*level=*/0) : t, false); };
   node->q = plain(q); node->k = plain(k); node->v = plain(v);
   const size_t n_out = dual ? 2 : 1;
   if (dual) {

@@ -114,3 +114,40 @@ def test_tangent_of_an_upstream_gradient_is_not_dropped_silently(ops):
     pull = lambda g: torch.func.vjp(lambda a: _call(ops, a, k, v), q)[1](g)[0]
     with pytest.raises(RuntimeError, match="not supported"):
         torch.func.jvp(pull, (go,), (tgo,))
+
+
+def _recorded(ops, how, ts):
+    """(outputs, tangent outputs) of a call whose q, k, v require a gradient, and nothing else does."""
+    q, k, v, tq, tk, tv = ts
+    if how == "plain":
+        return [_call(ops, q, k, v)]
+    if how == "dual":
+        return list(_dual(ops, *ts))
+    if how == "func_jvp":
+        return list(torch.func.jvp(lambda *x: _call(ops, *x), (q, k, v), (tq, tk, tv)))
+    with fwAD.dual_level():
+        return list(fwAD.unpack_dual(_call(ops, *(fwAD.make_dual(p, t) for p, t in ((q, tq), (k, tk), (v, tv))))))
+
+
+@pytest.mark.parametrize("how", ["plain", "dual", "func_jvp", "dual_level"])
+def test_differentiating_the_backward_raises(ops, how):
+    """``create_graph=True``: whichever way the call was recorded and with constant upstream gradients, the gradients are not
+    constants; differentiating them raises."""
+    ts = [t.requires_grad_(i < 3) for i, t in enumerate(_inputs(6, requires_grad=False))]
+    outs = _recorded(ops, how, ts)
+    grads = torch.autograd.grad(outs, ts[:3], [torch.ones_like(o) for o in outs], create_graph=True)
+    assert all(g.requires_grad for g in grads)
+    with pytest.raises(RuntimeError, match="differentiate twice"):
+        grads[0].square().sum().backward()
+
+
+@pytest.mark.parametrize("how", ["plain", "dual", "func_jvp", "dual_level"])
+def test_inputs_changed_in_place_are_noticed(ops, how):
+    """What the backward needs is saved with its version: an input that is changed before the backward raises."""
+    leaves = [t.requires_grad_(i < 3) for i, t in enumerate(_inputs(6, requires_grad=False))]
+    ts = [t * 1.0 if i < 3 else t for i, t in enumerate(leaves)]
+    outs = _recorded(ops, how, ts)
+    with torch.no_grad():
+        ts[1].add_(1.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(outs, leaves[:3], [torch.ones_like(o) for o in outs])
