@@ -283,8 +283,8 @@ const c10::TypedOperatorHandle<F>& op(const char* name) {
 
 // ------------------------------------------------------------------------------------------------ autograd
 struct AttentionBackward : public torch::autograd::Node {
-  SavedVariable q, k, v, tq, tk, tv, o, to, stats;
-  Tensor mask, summary;   // never differentiated; kept as they are
+  SavedVariable q, k, v, tq, tk, tv, o, to, stats, summary;
+  Tensor mask;   // the caller's, never differentiated: kept as it is
   bool dual = false, causal = false;
   double scale = 1.0, dropout_p = 0.0;
   int64_t dropout_seed = 0;
@@ -292,9 +292,8 @@ struct AttentionBackward : public torch::autograd::Node {
   std::string name() const override { return "JVPAttentionBackward"; }
   void release_variables() override {
     const std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable* s : {&q, &k, &v, &tq, &tk, &tv, &o, &to, &stats}) s->reset_data();
+    for (SavedVariable* s : {&q, &k, &v, &tq, &tk, &tv, &o, &to, &stats, &summary}) s->reset_data();
     mask.reset();
-    summary.reset();
   }
   // An output that the loss does not use arrives as an undefined gradient. Without one for the tangent output the
   // primal-only kernels run and the tangent inputs get no gradient.
@@ -309,7 +308,7 @@ struct AttentionBackward : public torch::autograd::Node {
     const std::vector<Tensor> g = op<BwdFn>("jvpfa::bwd").call(
         opt(go), opt(gto), q.unpack(), k.unpack(), v.unpack(), both ? opt(tq.unpack()) : OptTensor(),
         both ? opt(tk.unpack()) : OptTensor(), both ? opt(tv.unpack()) : OptTensor(), o.unpack(self),
-        both ? opt(to.unpack(self)) : OptTensor(), stats.unpack(), opt(mask), opt(summary), causal, scale, dropout_p, dropout_seed);
+        both ? opt(to.unpack(self)) : OptTensor(), stats.unpack(), opt(mask), opt(summary.unpack()), causal, scale, dropout_p, dropout_seed);
     for (size_t i = 0; i < g.size(); ++i)
       if (task_should_compute_output(i)) res[i] = g[i];
     return res;
@@ -347,7 +346,7 @@ std::vector<Tensor> fwd_autograd(const Tensor& q, const Tensor& k, const Tensor&
   node->stats = SavedVariable(out[n_out], false);
   if (mask.has_value() && mask->defined()) {
     node->mask = *mask;
-    node->summary = out[n_out + 1];
+    node->summary = SavedVariable(out[n_out + 1], false);
   }
   node->dual = dual; node->causal = causal; node->scale = scale;
   node->dropout_p = dropout_p; node->dropout_seed = dropout_seed;

@@ -151,3 +151,21 @@ def test_inputs_changed_in_place_are_noticed(ops, how):
         ts[1].add_(1.0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         torch.autograd.grad(outs, leaves[:3], [torch.ones_like(o) for o in outs])
+
+
+@pytest.mark.parametrize("dual", [False, True])
+def test_mask_summary_goes_through_saved_tensor_hooks(ops, dual):
+    """Everything of the size of the mask that the call makes is offered to saved-tensor hooks (offloading, checkpointing), and
+    the backward takes it from there."""
+    ts = _inputs(6)
+    mask = torch.ones(1, 1, N, N, dtype=torch.bool)
+    kept = []
+
+    def pack(t):
+        kept.append(t)
+        return len(kept) - 1
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda i: kept[i]):
+        outs = list(_dual(ops, *ts, mask=mask)) if dual else [_call(ops, *ts[:3], mask=mask)]
+    assert sum(t.dtype == torch.uint8 for t in kept) == 1
+    torch.autograd.grad(outs, ts[:3], [torch.ones_like(o) for o in outs])
