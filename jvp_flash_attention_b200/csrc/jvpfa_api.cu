@@ -20,6 +20,12 @@ TensorMapEncodeFn tensor_map_encoder() {
         q == cudaDriverEntryPointSuccess)
       fn = reinterpret_cast<TensorMapEncodeFn>(p);
   });
+  // The encoder is a driver call: it wants a context, which a thread without a CUDA runtime call so far does not have.
+  thread_local bool has_context = false;
+  if (!has_context) {
+    int dev = -1;
+    has_context = cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+  }
   return fn;
 }
 

@@ -49,3 +49,15 @@ def test_tangents_that_cannot_be_taken_raise(dev):
     inner = lambda x: torch.func.jvp(lambda y: JVPAttn.fwd_dual(y, q, q), (x,), (t,))[1]
     with pytest.raises(RuntimeError):
         torch.func.jvp(inner, (q,), (t,))
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float16, 64), (torch.bfloat16, 128), (torch.float16, 256), (torch.bfloat16, 256), (torch.float32, 64)])
+def test_first_cuda_work_of_a_thread(dev, dtype, D):
+    """A call may be the first thing that a thread does on the GPU."""
+    from concurrent.futures import ThreadPoolExecutor
+    from jvp_flash_attention_b200 import attention
+    q = torch.randn(1, 2, 128, D, device=dev, dtype=dtype)
+    want = attention(q, q, q)
+    with ThreadPoolExecutor(1) as thread:
+        got = thread.submit(attention, q, q, q).result()
+    assert torch.equal(got, want)
