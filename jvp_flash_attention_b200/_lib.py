@@ -258,8 +258,9 @@ def stream_ptr(device) -> C.c_void_p:
 
 # Workspaces (status word + scratch), one per (device, stream), grown on demand. Kernels of calls that share a
 # workspace must be ordered on one stream (the backward's per-row statistics live in it between its preprocess and
-# family kernels), so every stream gets its own. A buffer that is outgrown is kept alive until the process ends:
-# kernels already enqueued may still use it.
+# family kernels), so every stream gets its own; the library enqueues a call's kernels without another thread's on the
+# same workspace in between. A buffer that is outgrown is kept alive until the process ends: kernels already enqueued may
+# still use it.
 class _Workspace:
     def __init__(self, device, nbytes: int, before: "_Workspace | None"):
         self.buf = torch.zeros(nbytes, dtype=torch.uint8, device=device)
@@ -275,6 +276,7 @@ class _Workspace:
 
 
 _workspaces: dict = {}
+_workspace_lock = threading.Lock()
 
 
 def _ws_key(device):
@@ -294,13 +296,14 @@ def _raise_timeout(ws: _Workspace, device) -> None:
 
 def _workspace_object(device, key, nbytes: int) -> _Workspace:
     """Before handing the workspace of ``key`` out, looks at its status word on the host (no synchronisation): a
-    device-side wait that gave up in an earlier call raises here."""
-    ws = _workspaces.get(key)
-    if ws is not None and int(ws.host[0]) != 0:
-        _raise_timeout(ws, device)
-    if ws is None or ws.buf.numel() < nbytes:
-        _workspaces[key] = ws = _Workspace(device, max(nbytes, 1 << 20), ws)
-    return ws
+    device-side wait that gave up in an earlier call raises here. One thread at a time: allocating lets others run."""
+    with _workspace_lock:
+        ws = _workspaces.get(key)
+        if ws is not None and int(ws.host[0]) != 0:
+            _raise_timeout(ws, device)
+        if ws is None or ws.buf.numel() < nbytes:
+            _workspaces[key] = ws = _Workspace(device, max(nbytes, 1 << 20), ws)
+        return ws
 
 
 def workspace(device, nbytes: int) -> torch.Tensor:

@@ -497,6 +497,14 @@ int check_common(int B, int H, int N, int D, int dtype, int causal, const jvpfa_
   return JVPFA_OK;
 }
 
+// A call's kernels hand data to one another through its workspace (per-row statistics, split operands). Host threads may share a
+// stream and with it a workspace: the launches of one call are enqueued without another's on the same workspace in between. One
+// mutex per workspace, as far as 64 of them tell workspaces apart; nothing that it is held for waits for another thread.
+std::mutex& workspace_mutex(const void* workspace) {
+  static std::mutex mutexes[64];
+  return mutexes[(reinterpret_cast<uintptr_t>(workspace) >> 9) % 64];
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Input layouts: the tensor-core paths read strided views in place when TMA (16-bit inputs) or the split pre-pass
@@ -656,7 +664,8 @@ int jvpfa_fwd_status(const jvpfa_fwd_args* a, int32_t* status, void* stream) {
       !(sm100_split_path_supported(a->dtype, a->D, a->N) && a->workspace_bytes >= fwd_sm100_split_workspace_bytes(*a)))
     return JVPFA_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (sm100_path_supported(a->dtype, a->D, a->N)) return launch_fwd_sm100(*a, status, s);
+  if (sm100_path_supported(a->dtype, a->D, a->N)) return launch_fwd_sm100(*a, status, s);   // (one kernel, no scratch)
+  const std::lock_guard<std::mutex> lock(workspace_mutex(a->workspace));
   // fp32, and fp16 above head dimension 128: the tensor-core path when the workspace has room for the split operands, else the
   // CUDA-core kernels
   if (sm100_wide_path_supported(a->dtype, a->D, a->N) && a->workspace_bytes >= fwd_sm100_wide_workspace_bytes(*a))
@@ -712,6 +721,7 @@ int bwd_checked(const jvpfa_bwd_args* a, int* status, void* stream, void* const*
   LaunchMarks marks;
   marks.events = events;
   marks.stream = s;
+  const std::lock_guard<std::mutex> lock(workspace_mutex(eff.workspace));
   if (sm100_path_supported(eff.dtype, eff.D, eff.N)) return launch_bwd_sm100(eff, status, s, marks);
   // fp32, and fp16 above head dimension 128: the tensor-core path when the workspace has room for the split operands, else the
   // CUDA-core kernels

@@ -103,3 +103,28 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setenv("JVPFA_LIBRARY", str(tmp_path / "nope.so"))
     with pytest.raises(RuntimeError, match="no non-CUDA fallback"):
         _lib.lib()
+
+
+def test_one_workspace_per_stream_under_threads(monkeypatch):
+    """Threads that ask for the workspace of one stream at the same time get the same one: a second one would replace the first
+    while addresses of it are in use."""
+    import threading
+    import time
+    from jvp_flash_attention_b200 import _lib
+    made = []
+
+    class Slow:
+        def __init__(self, device, nbytes, before):
+            time.sleep(0.05)                       # (allocating lets other threads run)
+            self.buf, self.host = torch.zeros(nbytes, dtype=torch.uint8), torch.zeros(1, dtype=torch.int32)
+            made.append(self)
+
+    monkeypatch.setattr(_lib, "_Workspace", Slow)
+    monkeypatch.setattr(_lib, "_workspaces", {})
+    got = []
+    threads = [threading.Thread(target=lambda: got.append(_lib._workspace_object(torch.device("cuda", 0), (0, 7), 4096))) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(made) == 1 and all(w is made[0] for w in got)

@@ -61,3 +61,39 @@ def test_first_cuda_work_of_a_thread(dev, dtype, D):
     with ThreadPoolExecutor(1) as thread:
         got = thread.submit(attention, q, q, q).result()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("forward,backward", [
+    ((torch.float32, 64), (torch.float32, 64)), ((torch.float16, 256), (torch.bfloat16, 64)), ((torch.float32, 32), (torch.float16, 136)),
+])
+def test_two_threads_on_one_stream(dev, forward, backward):
+    """Forward calls of one thread against backward calls of another, on the same stream and therefore with the same scratch
+    (split operands, per-row statistics): each gives the bits it gives alone."""
+    import threading
+    from jvp_flash_attention_b200.jvp_attention import JVPAttn
+
+    def inputs(dtype, D, seed):
+        g = torch.Generator(device=dev).manual_seed(seed)
+        return [torch.randn(2, 4, 256, D, device=dev, generator=g).to(dtype) for _ in range(8)]
+
+    f = inputs(*forward, 1)
+    b = inputs(*backward, 2)
+    leaves = [t.requires_grad_() for t in b[:6]]
+    outs = JVPAttn.dual(*leaves, causal=True)
+    run_f = lambda: list(JVPAttn.dual(*f[:6]))
+    run_b = lambda: list(torch.autograd.grad(outs, leaves, b[6:], retain_graph=True))
+    want = [run_f(), run_b()]
+    got, start = [None, None], threading.Barrier(2)
+
+    def repeat(i, run):
+        start.wait()
+        got[i] = [run() for _ in range(60)]
+
+    threads = [threading.Thread(target=repeat, args=(i, run)) for i, run in enumerate((run_f, run_b))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for w, results in zip(want, got):
+        assert all(torch.equal(x, y) for r in results for x, y in zip(r, w))
