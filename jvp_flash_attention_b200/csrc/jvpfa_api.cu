@@ -645,6 +645,7 @@ int jvpfa_fwd_status(const jvpfa_fwd_args* a, int32_t* status, void* stream) {
   if (a == nullptr) return JVPFA_ERR_BAD_ARG;
   int rc = check_common(a->B, a->H, a->N, a->D, a->dtype, a->causal, a->mask, a->workspace, a->workspace_bytes, kStatusBytes);
   if (rc != JVPFA_OK) return rc;
+  if (status == nullptr) return JVPFA_ERR_BAD_ARG;   // (a wait that gives up writes there)
   if (!a->q || !a->k || !a->v || !a->o || !a->lse2 || !a->mu) return JVPFA_ERR_BAD_ARG;
   const bool dual = a->tq != nullptr;
   if (dual && (!a->tk || !a->tv || !a->to)) return JVPFA_ERR_BAD_ARG;
@@ -687,6 +688,7 @@ int bwd_checked(const jvpfa_bwd_args* a, int* status, void* stream, void* const*
   int rc = check_common(a->B, a->H, a->N, a->D, a->dtype, a->causal, a->mask, a->workspace, a->workspace_bytes,
                         sm100_path_supported(a->dtype, a->D, a->N) ? bwd_sm100_workspace_bytes(*a) : bwd_generic_workspace_bytes(*a));
   if (rc != JVPFA_OK) return rc;
+  if (status == nullptr) return JVPFA_ERR_BAD_ARG;   // (a wait that gives up writes there)
   if (!a->q || !a->k || !a->v || !a->o || !a->lse2 || !a->mu || !a->go || !a->dq || !a->dk || !a->dv) return JVPFA_ERR_BAD_ARG;
   const bool dual = a->tq != nullptr;   // tq == NULL: primal-only backward, the tangent-side pointers are ignored
   if (dual && (!a->tk || !a->tv || !a->to || !a->gto || !a->dtq || !a->dtk || !a->dtv)) return JVPFA_ERR_BAD_ARG;

@@ -128,3 +128,17 @@ def test_one_workspace_per_stream_under_threads(monkeypatch):
     for t in threads:
         t.join()
     assert len(made) == 1 and all(w is made[0] for w in got)
+
+
+def test_status_word_is_required(built_library):
+    """A call that is complete but for the status word, or for its tensors, is refused before anything is launched."""
+    from jvp_flash_attention_b200 import _lib
+    word = C.c_void_p(4096)
+    for args, fn, tensors in ((_lib.FwdArgs(), built_library.jvpfa_fwd_status, ("q", "k", "v", "o", "lse2", "mu")),
+                              (_lib.BwdArgs(), built_library.jvpfa_bwd_status, ("q", "k", "v", "o", "lse2", "mu", "go", "dq", "dk", "dv"))):
+        args.B, args.H, args.N, args.D, args.dtype = 1, 1, 64, 64, _lib.BF16
+        args.workspace, args.workspace_bytes = 4096, 1 << 20
+        assert fn(C.byref(args), word, None) == _lib.ERR_BAD_ARG       # no tensors
+        for n in tensors:
+            setattr(args, n, 4096)
+        assert fn(C.byref(args), None, None) == _lib.ERR_BAD_ARG       # no status word
