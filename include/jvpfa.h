@@ -171,10 +171,11 @@ int jvpfa_sm_clock_probe(float* mhz_out, int32_t duration_us, void* stream);
 
 /* Self-test of the failure-detection path. Launches one tiny kernel on `stream` in which a single thread waits, with
  * the kernels' own bounded wait, on a barrier that nothing arrives on: after `budget_us` microseconds (1 .. 1000000)
- * the wait gives up, writes 177 (100 + wait id 77) into the status word at the start of `workspace` and the kernel
+ * the wait gives up, writes 177 (100 + wait id 77) into the status word at `workspace` and the kernel
  * returns normally; a second wait in the same kernel takes the short path of an already failed CTA. `out4` (device,
- * four int32) receives the two wait results (0 = gave up) and their durations in microseconds. Afterwards
- * jvpfa_read_status reports JVPFA_ERR_DEVICE_TIMEOUT once. Nothing faults, traps or spins without bound. No reference
+ * four int32) receives the two wait results (0 = gave up) and their durations in microseconds. `workspace` is the start of
+ * a workspace (jvpfa_read_status then reports JVPFA_ERR_DEVICE_TIMEOUT once) or a status word of its own, as
+ * jvpfa_fwd_status takes one. Nothing faults, traps or spins without bound. No reference
  * counterpart (its errors are host-side Python exceptions, jvp_attention.py:2550, 2574, 3111). */
 int jvpfa_selftest_timeout(void* workspace, int32_t budget_us, int32_t* out4, void* stream);
 

@@ -264,7 +264,7 @@ def stream_ptr(device) -> C.c_void_p:
 class _Workspace:
     def __init__(self, device, nbytes: int, before: "_Workspace | None"):
         self.buf = torch.zeros(nbytes, dtype=torch.uint8, device=device)
-        self.word = self.buf[:4].view(torch.int32)                       # status word of the self-test
+        self.word = self.buf[:4].view(torch.int32)                       # status word of jvpfa_bwd_marked
         # status word of the attention kernels: pinned host memory they write to when a wait gives up, so that a call
         # neither copies it nor waits for it (the copy was 3 us of the stream and about as much host time a call)
         self.host = torch.zeros(1, dtype=torch.int32).pin_memory() if before is None else before.host
@@ -348,12 +348,11 @@ def selftest_timeout(device, budget_us: int = 2000) -> torch.Tensor:
     """Runs the library's failure-detection self-test on the current stream of ``device``: a bounded device-side wait
     that is made to run out. Returns the (4,) int32 device tensor with the two wait results and their durations in
     microseconds. The status word is then non-zero: the next call on this stream, or ``read_status``, raises."""
-    ws = workspace(device, 256)
+    ws = _workspace_object(device, _ws_key(device), 256)
     out = torch.full((4,), -1, dtype=torch.int32, device=device)
-    check(lib().jvpfa_selftest_timeout(C.c_void_p(ws.data_ptr()), int(budget_us), C.c_void_p(out.data_ptr()),
+    # the word that the attention kernels write to: pinned host memory
+    check(lib().jvpfa_selftest_timeout(C.c_void_p(ws.status_ptr), int(budget_us), C.c_void_p(out.data_ptr()),
                                        stream_ptr(device)))
-    w = _workspaces[_ws_key(device)]
-    w.host.copy_(w.word, non_blocking=True)      # the self-test writes to the workspace: where the next call looks is on the host
     return out
 
 

@@ -36,7 +36,7 @@ def test_next_call_on_the_stream_raises_without_synchronising(dev):
     q = torch.randn(1, 2, 128, 64, device=dev, dtype=torch.bfloat16)
     attention(q, q, q)                                      # makes sure the stream has a workspace
     _lib.selftest_timeout(dev, budget_us=2000)
-    torch.cuda.synchronize()                                # the status copy has landed in pinned host memory
+    torch.cuda.synchronize()                                # the status word in pinned host memory has been written
     with pytest.raises(_lib.JvpfaError) as err:
         attention(q, q, q)
     assert err.value.status == _lib.ERR_DEVICE_TIMEOUT
