@@ -215,6 +215,8 @@ int jvpfa_bwd_noalloc(const jvpfa_bwd_args* args, int32_t* status_word_out, void
  * The library keeps no state for this. No reference counterpart (the reference times whole calls with perf_counter,
  * tests/test_jvp_attention.py:116-143). */
 int jvpfa_bwd_marked(const jvpfa_bwd_args* args, void* stream, void* const* events, int32_t n_events);
+/* With the device status word at `status`, as jvpfa_bwd_status. */
+int jvpfa_bwd_marked_status(const jvpfa_bwd_args* args, int32_t* status, void* stream, void* const* events, int32_t n_events);
 
 #ifdef __cplusplus
 }

@@ -31,6 +31,7 @@ EXPORTED_SYMBOLS = (
     "jvpfa_bwd",
     "jvpfa_read_status",
     "jvpfa_bwd_marked",
+    "jvpfa_bwd_marked_status",
     "jvpfa_selftest_timeout",
     "jvpfa_sm_clock_probe",
     "jvpfa_bwd_noalloc",
@@ -133,6 +134,8 @@ def lib():
                 L.jvpfa_selftest_timeout.argtypes = [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p]
                 L.jvpfa_bwd_marked.restype = C.c_int
                 L.jvpfa_bwd_marked.argtypes = [C.POINTER(BwdArgs), C.c_void_p, C.POINTER(C.c_void_p), C.c_int32]
+                L.jvpfa_bwd_marked_status.restype = C.c_int
+                L.jvpfa_bwd_marked_status.argtypes = [C.POINTER(BwdArgs), C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p), C.c_int32]
                 L.jvpfa_fwd_status.restype = C.c_int
                 L.jvpfa_fwd_status.argtypes = [C.POINTER(FwdArgs), C.c_void_p, C.c_void_p]
                 L.jvpfa_bwd_status.restype = C.c_int
@@ -264,7 +267,7 @@ def stream_ptr(device) -> C.c_void_p:
 class _Workspace:
     def __init__(self, device, nbytes: int, before: "_Workspace | None"):
         self.buf = torch.zeros(nbytes, dtype=torch.uint8, device=device)
-        self.word = self.buf[:4].view(torch.int32)                       # status word of jvpfa_bwd_marked
+        self.word = self.buf[:4].view(torch.int32)                       # status word of calls without one of their own
         # status word of the attention kernels: pinned host memory they write to when a wait gives up, so that a call
         # neither copies it nor waits for it (the copy was 3 us of the stream and about as much host time a call)
         self.host = torch.zeros(1, dtype=torch.int32).pin_memory() if before is None else before.host
@@ -440,5 +443,5 @@ def bwd(q, k, v, tq, tk, tv, o, to, lse2, mu, go, gto, mask_c: Mask, summary, ca
         check(lib().jvpfa_bwd_status(C.byref(a), C.c_void_p(ws.status_ptr), stream_ptr(q.device)))
     else:
         handles = (C.c_void_p * 5)(*[C.c_void_p(e.cuda_event) for e in marks])
-        check(lib().jvpfa_bwd_marked(C.byref(a), stream_ptr(q.device), handles, 5))
+        check(lib().jvpfa_bwd_marked_status(C.byref(a), C.c_void_p(ws.status_ptr), stream_ptr(q.device), handles, 5))
     return tuple(outs)

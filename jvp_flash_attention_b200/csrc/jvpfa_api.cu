@@ -750,10 +750,14 @@ int jvpfa_bwd_status(const jvpfa_bwd_args* a, int32_t* status, void* stream) {
 }
 
 int jvpfa_bwd_marked(const jvpfa_bwd_args* a, void* stream, void* const* events, int32_t n_events) {
+  return a == nullptr ? JVPFA_ERR_BAD_ARG : jvpfa_bwd_marked_status(a, static_cast<int32_t*>(a->workspace), stream, events, n_events);
+}
+
+int jvpfa_bwd_marked_status(const jvpfa_bwd_args* a, int32_t* status, void* stream, void* const* events, int32_t n_events) {
   if (events == nullptr || n_events != 5) return JVPFA_ERR_BAD_ARG;
   for (int i = 0; i < 5; ++i)
     if (events[i] == nullptr) return JVPFA_ERR_BAD_ARG;
-  return a == nullptr ? JVPFA_ERR_BAD_ARG : bwd_checked(a, static_cast<int*>(a->workspace), stream, events);
+  return a == nullptr ? JVPFA_ERR_BAD_ARG : bwd_checked(a, status, stream, events);
 }
 
 int jvpfa_sm_clock_probe(float* mhz_out, int32_t duration_us, void* stream) {

@@ -46,6 +46,33 @@ def test_next_call_on_the_stream_raises_without_synchronising(dev):
     assert torch.isfinite(o).all()
 
 
+def test_every_launch_reports_to_the_host_word(dev, monkeypatch):
+    """Forward, backward and the backward with events between its parts are given the status word that the next call looks at."""
+    from jvp_flash_attention_b200 import _lib
+    q, k, v, tq, tk, tv, go, gto = (torch.randn(1, 2, 128, 64, device=dev, dtype=torch.bfloat16) for _ in range(8))
+    m = _lib.make_mask(None, 1, 2, 128)
+    events = [torch.cuda.Event(enable_timing=True) for _ in range(5)]
+    for e in events:
+        e.record()
+    L, given = _lib.lib(), []
+
+    class Seen:
+        def __getattr__(self, name):
+            fn = getattr(L, name)
+            if name in ("jvpfa_fwd", "jvpfa_bwd", "jvpfa_bwd_marked"):
+                given.append(None)                        # (would report to the workspace)
+            if name in ("jvpfa_fwd_status", "jvpfa_bwd_status", "jvpfa_bwd_marked_status"):
+                return lambda a, status, *rest: (given.append(status.value), fn(a, status, *rest))[1]
+            return fn
+
+    monkeypatch.setattr(_lib, "lib", lambda: Seen())
+    o, to, lse2, mu = _lib.fwd(q, k, v, tq, tk, tv, m, None, False, 0.125)
+    for marks in (None, events):
+        _lib.bwd(q, k, v, tq, tk, tv, o, to, lse2, mu, go, gto, m, None, False, 0.125, marks=marks)
+    torch.cuda.synchronize()
+    assert given == [_lib._workspaces[_lib._ws_key(dev)].status_ptr] * 3
+
+
 def test_streams_have_their_own_workspace(dev):
     """Two backward calls on different streams must not share scratch (the per-row statistics live in it)."""
     from jvp_flash_attention_b200 import _lib
