@@ -461,8 +461,7 @@ def run_cuda(args, rank, world, local_rank):
             acc[nme] += marks[i][j].elapsed_time(marks[i][j + 1])
     kernels = {nme: {"ms_per_launch": acc[nme] / args.steps, "launches": args.steps} for nme in names}
     lfwd_f, lbwd_f = algorithmic_flops(1, U, N, D, causal)            # this rank's slice
-    # main backward launches of a step: one for all families, three from twenty waves of blocks per family on (bwd_sm100.cuh)
-    bwd_launches = 3 if causal and U * ((N + 127) // 128) >= 20 * 148 else 1
+    bwd_launches = 1     # main backward launches of a step: all families together
     fam_ms = (acc["bwd_q"] + acc["bwd_k"] + acc["bwd_v"]) / (3.0 * args.steps)
     # dominant kernel: the backward kernel, one launch per step; this pass runs its three families as launches of their own,
     # between events; algorithmic FLOPs per

@@ -912,7 +912,7 @@ struct BwdFamilies {
 // (B=8 H=16 N=4096 D=128 causal 8.4 ms instead of 5.0).
 // Measured against one launch per family (us): B=4 H=8 N=1024 D=128 causal fp16 primal only 102 -> 80; B=32 H=16 N=256 D=72
 // 285 -> 266; B=5 H=7 N=777 D=96 padded 156 -> 126; H=12 N=1024 D=128 94 -> 73; B=4 H=16 N=2048 D=64 694 -> 659; fp32 B=2 H=4
-// N=128 31 -> 12, B=2 H=12 N=2048 692 -> 632. launch_families has the one rule for a launch per family.
+// N=128 31 -> 12, B=2 H=12 N=2048 692 -> 632.
 template <int D, bool BF16, bool PAD, bool DUAL, bool SPLIT = false, bool DROP = false>
 __global__ void __launch_bounds__(352, 1) bwd_sm100_kernel(const __grid_constant__ BwdMaps maps, const __grid_constant__ BwdKParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -1068,12 +1068,11 @@ int launch_families(const jvpfa_bwd_args& a, const BwdMaps& maps, const float4* 
     return cudaGetLastError() == cudaSuccess;
   };
   marks.mark(1);
-  // One launch per family also where a family alone keeps the chip busy and its blocks differ in length, so that there is no
-  // empty wave to fill and only the alternation at the seams is left: causal, D > 64, from twenty waves of blocks on (backward,
-  // us, apart / together: B=8 H=16 N=4096 D=128 causal 5853 / 5905, fp16 6058 / 6113; B=4 2939 / 2954, B=2 1495 / 1472;
-  // B=8 N=2048 1765 / 1743; not causal 10602 / 10462; D=64 causal 3296 / 3282). A grid has at most 2^31 - 1 blocks.
-  const int64_t per_fam = static_cast<int64_t>(p.n_rt) * p.n_units;
-  const bool apart = (D > 64 && !SPLIT && p.causal && per_fam >= 20 * 148) || F::COUNT * per_fam > 0x7FFFFFFF;
+  // One launch per family also where the families together have more blocks than a grid can. Not for speed: where a family alone
+  // fills the chip neither form is the faster one (causal, us, apart / together, medians of three: B=8 H=16 N=4096 D=128 bf16
+  // 5484 / 5593, fp16 5900 / 5802, primal only 2932 / 2900; B=16 N=2048 3358 / 3414; B=32 N=1024 2125 / 2104; D=96 B=64 N=512
+  // 1471 / 1449; D=80 B=12 N=4096 7624 / 7696).
+  const bool apart = F::COUNT * static_cast<int64_t>(p.n_rt) * p.n_units > 0x7FFFFFFF;
   if (marks.events == nullptr && !apart) {
     if (!launch(0, F::COUNT)) return JVPFA_ERR_LAUNCH;
   } else {
