@@ -159,7 +159,8 @@ struct BwdCfg {
 // DROP: the forward applied dropout to the probabilities that multiply V, tV (dropout.cuh). The same keep pattern is
 // regenerated here: it scales X and A (the gradients that arrive through V, tV) in families Q, K, and P, tP (the operands
 // of dV, dtV) in family V; Delta and a come from the dropped-out O, tO and need no change.
-template <int D, int FAM, bool BF16, bool PAD, bool DUAL, bool SPLIT = false, bool DROP = false>
+// ELEMS: the mask may have to be read element by element.
+template <int D, int FAM, bool BF16, bool PAD, bool DUAL, bool SPLIT, bool DROP, bool ELEMS>
 __device__ __forceinline__ void bwd_family(const BwdMaps& maps, const BwdKParams& p, const int rt, const int bh, uint8_t* smem) {
   using C = BwdCfg<D, FAM, SPLIT>;
   constexpr int NA = C::NA, NB = C::NB;
@@ -594,7 +595,7 @@ __device__ __forceinline__ void bwd_family(const BwdMaps& maps, const BwdKParams
           const float other = p.mv.kind == JVPFA_MASK_BOOL ? -INFINITY : mask_tile_value(p.mv, b, h, my_qt, my_kt) * 1.4426950408889634f;
           mask_apply_bits(x2, (FAM == FAM_Q) ? mask_row_bits(p.mv, b, h, gr_c, j, wg) : mask_col_bits(p.mv, b, h, j, gr_c, wg), other);
         }
-        const bool mask_elems = mask_mode == 2;
+        const bool mask_elems = ELEMS && mask_mode == 2;
         // (keys past the end of the sequence: zero bits of a boolean mask already exclude them)
         if (need_causal || (need_bound && !(mask_mode == 1 && p.mv.kind == JVPFA_MASK_BOOL)) || mask_elems) {
 #pragma unroll
@@ -913,15 +914,15 @@ struct BwdFamilies {
 // Measured against one launch per family (us): B=4 H=8 N=1024 D=128 causal fp16 primal only 102 -> 80; B=32 H=16 N=256 D=72
 // 285 -> 266; B=5 H=7 N=777 D=96 padded 156 -> 126; H=12 N=1024 D=128 94 -> 73; B=4 H=16 N=2048 D=64 694 -> 659; fp32 B=2 H=4
 // N=128 31 -> 12, B=2 H=12 N=2048 692 -> 632.
-template <int D, bool BF16, bool PAD, bool DUAL, bool SPLIT = false, bool DROP = false>
+template <int D, bool BF16, bool PAD, bool DUAL, bool SPLIT, bool DROP, bool ELEMS>
 __global__ void __launch_bounds__(352, 1) bwd_sm100_kernel(const __grid_constant__ BwdMaps maps, const __grid_constant__ BwdKParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   using F = BwdFamilies<D, SPLIT>;
   const int per_fam = p.n_rt * p.n_units, idx = static_cast<int>(blockIdx.x) / per_fam, fam = p.first_fam + idx;
   const BlockWork work = block_work(static_cast<int>(blockIdx.x) - idx * per_fam, p.n_rt, p.n_units, p.unit_group, p.causal && fam == 1);
-  if (fam == 0) bwd_family<D, F::FAM[0], BF16, PAD, DUAL, SPLIT, DROP>(maps, p, work.tile, work.unit, smem);
-  else if (fam == 1) bwd_family<D, FAM_Q, BF16, PAD, DUAL, SPLIT, DROP>(maps, p, work.tile, work.unit, smem);
-  else if constexpr (F::COUNT == 3) bwd_family<D, FAM_V, BF16, PAD, DUAL, SPLIT, DROP>(maps, p, work.tile, work.unit, smem);
+  if (fam == 0) bwd_family<D, F::FAM[0], BF16, PAD, DUAL, SPLIT, DROP, ELEMS>(maps, p, work.tile, work.unit, smem);
+  else if (fam == 1) bwd_family<D, FAM_Q, BF16, PAD, DUAL, SPLIT, DROP, ELEMS>(maps, p, work.tile, work.unit, smem);
+  else if constexpr (F::COUNT == 3) bwd_family<D, FAM_V, BF16, PAD, DUAL, SPLIT, DROP, ELEMS>(maps, p, work.tile, work.unit, smem);
 }
 
 // Where the rows of the upstream gradients start: go and gto may be strided views, o and to are contiguous.
@@ -1041,7 +1042,7 @@ __global__ void bwd_preprocess_f32_kernel(const float* __restrict__ o, const flo
 // `a` holds the operands the tensor maps are built on: in the split-fp32 mode (SPLIT) the bf16 hi/lo tensors of the
 // pre-pass with 128 columns, and `real_D` is the head dimension of the outputs.
 // With events (`marks`) every family is a launch of its own between two of them, in the order Q, K, V (Q, KV).
-template <int D, bool BF16, bool PAD, bool DUAL, bool SPLIT = false, bool DROP = false>
+template <int D, bool BF16, bool PAD, bool DUAL, bool SPLIT, bool DROP, bool ELEMS>
 int launch_families(const jvpfa_bwd_args& a, const BwdMaps& maps, const float4* stats, int* status, cudaStream_t stream,
                     const LaunchMarks& marks, int real_D) {
   using F = BwdFamilies<D, SPLIT>;
@@ -1058,7 +1059,7 @@ int launch_families(const jvpfa_bwd_args& a, const BwdMaps& maps, const float4* 
   p.n_rt = (a.N + 127) / 128;
   p.n_units = a.B * a.H;
   p.unit_group = unit_group_size(p.n_units);
-  auto kern = bwd_sm100_kernel<D, BF16, PAD, DUAL, SPLIT, DROP>;
+  auto kern = bwd_sm100_kernel<D, BF16, PAD, DUAL, SPLIT, DROP, ELEMS>;
   const size_t smem = F::smem_bytes();
   static SmemOptIn opt_in;
   if (!opt_in.set(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_LAUNCH;
@@ -1109,17 +1110,22 @@ int launch_all(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, const 
   if (rc0 != JVPFA_OK) return rc0;
   BwdMaps maps;
   if (!maps.encode(a)) return JVPFA_ERR_LAUNCH;
-  auto three = [&](auto pad, auto dual, auto drop) {
-    return launch_families<D, BF16, decltype(pad)::value, decltype(dual)::value, false, decltype(drop)::value>(a, maps, stats, status, stream,
-                                                                                                               marks, a.D);
+  auto go = [&](auto pad, auto dual, auto drop, auto elems) {
+    return launch_families<D, BF16, decltype(pad)::value, decltype(dual)::value, false, decltype(drop)::value, decltype(elems)::value>(
+        a, maps, stats, status, stream, marks, a.D);
   };
-  const bool dual = a.tq != nullptr;
-  if (a.dropout_p > 0.f) {
-    if (a.D == D) return dual ? three(std::false_type{}, std::true_type{}, std::true_type{}) : three(std::false_type{}, std::false_type{}, std::true_type{});
-    return dual ? three(std::true_type{}, std::true_type{}, std::true_type{}) : three(std::true_type{}, std::false_type{}, std::true_type{});
-  }
-  if (a.D == D) return dual ? three(std::false_type{}, std::true_type{}, std::false_type{}) : three(std::false_type{}, std::false_type{}, std::false_type{});
-  return dual ? three(std::true_type{}, std::true_type{}, std::false_type{}) : three(std::true_type{}, std::false_type{}, std::false_type{});
+  auto by_mask = [&](auto pad, auto dual, auto drop) {
+    // Boolean masks with a summary never read the mask element by element. Without that code (bf16, B=2 H=8 N=1024, us) 94 -> 85
+    // at D=64, 134 -> 124 at D=128. Calls without a mask stay on the kernels that have it: B=4 H=16 N=2048 D=64 679 with, 689
+    // without (its registers spill), primal only 454 and 443.
+    const bool packed = a.mask.kind == JVPFA_MASK_BOOL && a.mask_summary != nullptr;
+    return packed ? go(pad, dual, drop, std::false_type{}) : go(pad, dual, drop, std::true_type{});
+  };
+  auto by_drop = [&](auto pad, auto dual) {
+    return a.dropout_p > 0.f ? by_mask(pad, dual, std::true_type{}) : by_mask(pad, dual, std::false_type{});
+  };
+  auto by_dual = [&](auto pad) { return a.tq != nullptr ? by_drop(pad, std::true_type{}) : by_drop(pad, std::false_type{}); };
+  return a.D == D ? by_dual(std::false_type{}) : by_dual(std::true_type{});
 }
 
 // fp32 inputs: statistics from the fp32 tensors, split pre-pass of the eight (primal-only: four) MMA operands into the
@@ -1158,7 +1164,7 @@ int launch_split(const jvpfa_bwd_args& a, int* status, cudaStream_t stream, cons
   if (DUAL) { m.tq = dst[4]; m.tk = dst[5]; m.tv = dst[6]; m.gto = dst[7]; }
   BwdMaps maps;
   if (!maps.encode(m)) return JVPFA_ERR_LAUNCH;
-  return launch_families<128, true, false, DUAL, true, DROP>(m, maps, stats, status, stream, marks, a.D);
+  return launch_families<128, true, false, DUAL, true, DROP, true>(m, maps, stats, status, stream, marks, a.D);
 }
 
 }  // namespace

@@ -188,8 +188,7 @@ __device__ __forceinline__ void mask_bias_run(float (&bias)[CNT], const MaskView
     } else if (!along_k && mv.dtype != JVPFA_F32 && first + CNT <= N) {
       // down a column: all loads are issued before the first value is used (with the type and the bound looked at entry by entry
       // they ran one after the other: additive bf16 mask, B=2 H=8 N=1024, backward 141 -> 107 us at D = 64, 256 -> 165 us at 128).
-      // Rows that are not aligned, fp32 masks and the last tile stay on the short code below: unrolling those as well made
-      // boolean masks, which never get here, pay for the larger kernels (74 -> 80 us; 78 us like this).
+      // Rows that are not aligned, fp32 masks and the last tile stay on the short code below.
       uint32_t raw[CNT];
 #pragma unroll
       for (int i = 0; i < CNT; ++i, mp += 2 * step) raw[i] = __ldg(reinterpret_cast<const uint16_t*>(mp));
