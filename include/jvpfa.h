@@ -153,7 +153,8 @@ int jvpfa_bwd_status(const jvpfa_bwd_args* args, int32_t* status, void* stream);
 /* The reference's mask check (jvp_attention.py:2632-2656) from the summary of the mask instead of two more passes over it.
  * `begin` launches it behind the summary pre-pass on the same stream; `end` waits for that launch alone (kernels launched
  * in between keep running) and writes 0 (fine), 1 (a boolean mask has a (batch, head) plane with nothing kept) or 2 (an
- * additive mask holds a NaN) to `verdict`. `end` must be called exactly once per successful `begin`. */
+ * additive mask holds a NaN) to `verdict`. `end` must be called exactly once per successful `begin`. `begin` answers
+ * JVPFA_ERR_LAUNCH on a stream that is being captured. */
 int jvpfa_mask_check_begin(const jvpfa_mask* mask, int32_t B, int32_t H, int32_t N, const uint8_t* summary, void* stream, void** check);
 int jvpfa_mask_check_end(void* check, int32_t* verdict);
 

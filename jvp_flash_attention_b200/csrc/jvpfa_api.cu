@@ -3,6 +3,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <vector>
 #include "host_common.h"
 #include "mask_common.cuh"
@@ -432,6 +433,7 @@ void free_mask_check(MaskCheck* c) {
   if (c->done != nullptr) cudaEventDestroy(c->done);
   if (c->verdict != nullptr) cudaFreeHost(c->verdict);
   delete c;
+  (void)cudaGetLastError();   // (called after a failure: the next launch must not report it)
 }
 MaskCheck* take_mask_check() {
   int dev = -1;
@@ -445,7 +447,8 @@ MaskCheck* take_mask_check() {
         return c;
       }
   }
-  MaskCheck* c = new MaskCheck;
+  MaskCheck* c = new (std::nothrow) MaskCheck;
+  if (c == nullptr) return nullptr;
   c->device = dev;
   if (cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming) != cudaSuccess ||
       cudaHostAlloc(reinterpret_cast<void**>(&c->verdict), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
@@ -609,6 +612,12 @@ int jvpfa_mask_summary(const jvpfa_mask* mask, int32_t B, int32_t H, int32_t N, 
 int jvpfa_mask_check_begin(const jvpfa_mask* mask, int32_t B, int32_t H, int32_t N, const uint8_t* summary, void* stream, void** check) {
   if (mask == nullptr || summary == nullptr || check == nullptr || B <= 0 || H <= 0 || N <= 0) return JVPFA_ERR_BAD_ARG;
   *check = nullptr;
+  // `end` waits on the host, which a capture cannot contain: refused here, before the capture is spoilt
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return JVPFA_ERR_LAUNCH;
+  }
   MaskCheck* c = take_mask_check();
   if (c == nullptr) return JVPFA_ERR_LAUNCH;
   *c->verdict = 0;

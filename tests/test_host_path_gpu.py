@@ -97,3 +97,26 @@ def test_two_threads_on_one_stream(dev, forward, backward):
     torch.cuda.synchronize()
     for w, results in zip(want, got):
         assert all(torch.equal(x, y) for r in results for x, y in zip(r, w))
+
+
+def test_mask_check_inside_a_capture(dev):
+    """The verdict is read on the host: refused while a graph is captured, without spoiling the capture or the calls after it;
+    without the check a masked call can be captured."""
+    from jvp_flash_attention_b200 import attention
+    q = torch.randn(1, 2, 130, 64, device=dev, dtype=torch.float16)
+    mask = torch.rand(1, 1, 130, 130, device=dev) < 0.9
+    want = attention(q, q, q, attn_mask=mask)
+    stream = torch.cuda.Stream(dev)
+    stream.wait_stream(torch.cuda.current_stream(dev))
+    with torch.cuda.stream(stream):
+        attention(q, q, q, attn_mask=mask)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        with pytest.raises(RuntimeError):
+            attention(q, q, q, attn_mask=mask)
+        got = attention(q, q, q, attn_mask=mask, verify_attn_mask=False)
+    assert torch.equal(attention(q, q, q, attn_mask=mask), want)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
