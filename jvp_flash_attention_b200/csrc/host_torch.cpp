@@ -325,6 +325,7 @@ std::vector<Tensor> fwd_autograd(const Tensor& q, const Tensor& k, const Tensor&
   // tangents_taken: the caller has read the tangents of q, k, v at this level and passes them as tq, tk, tv
   if ((!tangents_taken && (has_fw_grad(q) || has_fw_grad(k) || has_fw_grad(v))) || has_fw_grad(tq) || has_fw_grad(tk) || has_fw_grad(tv))
     TORCH_CHECK_NOT_IMPLEMENTED(false, kNoNesting);
+  if (has_fw_grad(mask)) TORCH_CHECK_NOT_IMPLEMENTED(false, "JVP attention: a forward-mode tangent of the attention mask is not supported");
   const Tensor none;
   const bool record = torch::autograd::compute_requires_grad(q, k, v, dual ? *tq : none, dual ? *tk : none, dual ? *tv : none);
   std::vector<Tensor> out;

@@ -15,7 +15,7 @@ def _scores(q, k, tq, tk, mask, causal, scale):
     if causal:
         s = s.masked_fill(torch.ones(s.shape[-2:], dtype=torch.bool).triu(1), float("-inf"))
     if mask is not None:
-        s = s.masked_fill(~mask, float("-inf"))
+        s = s.masked_fill(~mask, float("-inf")) if mask.dtype == torch.bool else s + mask
     ts = None if tq is None else (tq @ k.transpose(-1, -2) + q @ tk.transpose(-1, -2)) * scale
     return s.softmax(-1), ts
 
@@ -169,3 +169,18 @@ def test_mask_summary_goes_through_saved_tensor_hooks(ops, dual):
         outs = list(_dual(ops, *ts, mask=mask)) if dual else [_call(ops, *ts[:3], mask=mask)]
     assert sum(t.dtype == torch.uint8 for t in kept) == 1
     torch.autograd.grad(outs, ts[:3], [torch.ones_like(o) for o in outs])
+
+
+@pytest.mark.parametrize("how", ["plain", "dual_level", "func_jvp", "dual"])
+def test_tangent_of_the_mask_is_refused(ops, how):
+    """The tangent of an additive mask is not part of what the kernels compute: refused instead of left out."""
+    q, k, v, tq, tk, tv = _inputs(6, requires_grad=False)
+    mask, tm = torch.zeros(1, 1, N, N), torch.ones(1, 1, N, N)
+    with pytest.raises(RuntimeError, match="not supported"):
+        if how == "func_jvp":
+            torch.func.jvp(lambda a, m: _call(ops, a, k, v, mask=m), (q, mask), (tq, tm))
+        with fwAD.dual_level():
+            m = fwAD.make_dual(mask, tm)
+            if how == "dual":
+                _dual(ops, q, k, v, tq, tk, tv, mask=m)
+            _call(ops, fwAD.make_dual(q, tq) if how == "dual_level" else q, k, v, mask=m)
