@@ -301,7 +301,9 @@ struct AttentionBackward : public torch::autograd::Node {
     const std::lock_guard<std::mutex> lock(mutex_);
     variable_list res(dual ? 6 : 3);
     const Tensor go = grads[0], gto = dual ? grads[1] : Tensor();
-    if (!go.defined() && !gto.defined()) return res;
+    bool wanted = false;
+    for (size_t i = 0; i < res.size(); ++i) wanted |= task_should_compute_output(i);
+    if (!wanted || (!go.defined() && !gto.defined())) return res;
     auto self = getptr();
     const bool both = gto.defined();
     const auto opt = [](const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); };
@@ -327,7 +329,9 @@ std::vector<Tensor> fwd_autograd(const Tensor& q, const Tensor& k, const Tensor&
     TORCH_CHECK_NOT_IMPLEMENTED(false, kNoNesting);
   if (has_fw_grad(mask)) TORCH_CHECK_NOT_IMPLEMENTED(false, "JVP attention: a forward-mode tangent of the attention mask is not supported");
   const Tensor none;
-  const bool record = torch::autograd::compute_requires_grad(q, k, v, dual ? *tq : none, dual ? *tk : none, dual ? *tv : none);
+  // (a mask that requires a gradient gets none, but the outputs can be differentiated)
+  const bool record = torch::autograd::compute_requires_grad(q, k, v, dual ? *tq : none, dual ? *tk : none, dual ? *tv : none,
+                                                             has(mask) ? *mask : none);
   std::vector<Tensor> out;
   {
     at::AutoDispatchBelowADInplaceOrView guard;

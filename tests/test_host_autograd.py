@@ -184,3 +184,12 @@ def test_tangent_of_the_mask_is_refused(ops, how):
             if how == "dual":
                 _dual(ops, q, k, v, tq, tk, tv, mask=m)
             _call(ops, fwAD.make_dual(q, tq) if how == "dual_level" else q, k, v, mask=m)
+
+
+def test_mask_that_requires_a_gradient(ops):
+    """It gets none, and a loss on the outputs can be differentiated all the same when nothing else requires a gradient."""
+    q, k, v, tq, tk, tv = _inputs(6, requires_grad=False)
+    mask = torch.zeros(1, 1, N, N, requires_grad=True)
+    for outs in ([_call(ops, q, k, v, mask=mask)], list(_dual(ops, q, k, v, tq, tk, tv, mask=mask))):
+        sum(o.sum() for o in outs).backward()
+        assert mask.grad is None
