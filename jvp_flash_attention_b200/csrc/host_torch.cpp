@@ -341,8 +341,7 @@ std::vector<Tensor> fwd_autograd(const Tensor& q, const Tensor& k, const Tensor&
   std::shared_ptr<AttentionBackward> node(new AttentionBackward(), torch::autograd::deleteNode);
   if (dual) node->set_next_edges(torch::autograd::collect_next_edges(q, k, v, *tq, *tk, *tv));
   else node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
-  // (without the tangent but with its place in the graph, which is what tells bwd_autograd that the gradients depend on it)
-  const auto plain = [&](const Tensor& t) { return SavedVariable(tangents_taken && has_fw_grad(t) ? t._fw_primal(/*level=*/0) : t, false); };
+  const auto plain = [&](const Tensor& t) { return SavedVariable(tangents_taken && has_fw_grad(t) ? t.detach() : t, false); };
   node->q = plain(q); node->k = plain(k); node->v = plain(v);
   const size_t n_out = dual ? 2 : 1;
   if (dual) {
@@ -384,11 +383,12 @@ std::vector<Tensor> bwd_autograd(const OptTensor& go_, const OptTensor& gto_, co
   }
   const Tensor none;
   const auto t = [&](const OptTensor& x) { return has(x) ? *x : none; };
-  if (torch::autograd::compute_requires_grad(t(go), t(gto), q, k, v, t(tq), t(tk), t(tv))) {
+  // (o: recorded whenever the gradients are of a recorded call; q, k, v of a call on dual tensors are saved without their graph)
+  if (torch::autograd::compute_requires_grad(t(go), t(gto), q, k, v, t(tq), t(tk), t(tv), o)) {
     // the gradients come from kernels: differentiating them again raises instead of returning zeros
     std::shared_ptr<torch::autograd::Node> err(
         new torch::autograd::Error("trying to differentiate twice: the gradients of JVP attention are computed by kernels",
-                                   torch::autograd::collect_next_edges(t(go), t(gto), q, k, v, t(tq), t(tk), t(tv))),
+                                   torch::autograd::collect_next_edges(t(go), t(gto), q, k, v, t(tq), t(tk), t(tv), o)),
         torch::autograd::deleteNode);
     for (Tensor& g : out) torch::autograd::set_history(g, err);
   }
