@@ -1069,10 +1069,10 @@ int launch_families(const jvpfa_bwd_args& a, const BwdMaps& maps, const float4* 
     return cudaGetLastError() == cudaSuccess;
   };
   marks.mark(1);
-  // One launch per family also where the families together have more blocks than a grid can. Not for speed: where a family alone
-  // fills the chip neither form is the faster one (causal, us, apart / together, medians of three: B=8 H=16 N=4096 D=128 bf16
-  // 5484 / 5593, fp16 5900 / 5802, primal only 2932 / 2900; B=16 N=2048 3358 / 3414; B=32 N=1024 2125 / 2104; D=96 B=64 N=512
-  // 1471 / 1449; D=80 B=12 N=4096 7624 / 7696).
+  // One launch per family also where the families together have more blocks than a grid can. Not for speed, also where a family
+  // alone fills the chip (causal, H=16, us, apart / together, 24 calls of each in turn: B=8 N=4096 D=128 bf16 5760 / 5821, fp16
+  // 6172 / 6213, primal only 3048 / 2988; B=4 2964 / 2940; B=2 1565 / 1505; B=16 N=2048 3488 / 3463; B=32 N=1024 2323 / 2285;
+  // B=64 N=512 1627 / 1575; B=4 N=8192 10816 / 10803; but B=8 N=4096 D=96 5406 / 5561, D=72 5252 / 5325).
   const bool apart = F::COUNT * static_cast<int64_t>(p.n_rt) * p.n_units > 0x7FFFFFFF;
   if (marks.events == nullptr && !apart) {
     if (!launch(0, F::COUNT)) return JVPFA_ERR_LAUNCH;
