@@ -120,3 +120,36 @@ def test_mask_check_inside_a_capture(dev):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("own_streams", [False, True])
+def test_mask_checks_on_two_threads(dev, own_streams):
+    """Verdicts of masks that are checked at the same time reach the calls they belong to."""
+    import threading
+    from jvp_flash_attention_b200 import attention
+    q = torch.randn(2, 2, 130, 64, device=dev, dtype=torch.float16)
+    good = torch.rand(2, 1, 130, 130, device=dev) < 0.9
+    bad = good.clone()
+    bad[1] = False
+    want = attention(q, q, q, attn_mask=good)
+    torch.cuda.synchronize()
+    wrong = []
+
+    def repeat(first):
+        with torch.cuda.stream(torch.cuda.Stream(dev) if own_streams else torch.cuda.current_stream(dev)):
+            for i in range(50):
+                try:
+                    ok = (i + first) % 2 == 0 and torch.equal(attention(q, q, q, attn_mask=good), want)
+                    if (i + first) % 2 == 1:
+                        attention(q, q, q, attn_mask=bad)
+                except AssertionError:
+                    ok = (i + first) % 2 == 1
+                if not ok:
+                    wrong.append(i)
+
+    threads = [threading.Thread(target=repeat, args=(f,)) for f in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
