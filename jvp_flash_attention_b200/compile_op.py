@@ -3,8 +3,8 @@
 Counterpart of the reference's ``jvp_flash_attention::attn_fwd_dual_triton`` custom op and its fake
 (jvp_flash_attention/jvp_attention.py:2247-2427), extended with a registered backward: the reference's compiled
 path has no autograd (its op is called under ``no_grad``, :2677-2692), here gradients flow through both outputs.
-``JVPAttn.dual`` switches to these operators while a graph is being compiled; eager calls keep using the
-``autograd.Function`` in ``jvp_attention.py``.
+``JVPAttn.dual`` switches to these operators while a graph is being compiled; eager calls go through the native host
+path (``csrc/host_torch.cpp``).
 """
 from __future__ import annotations
 

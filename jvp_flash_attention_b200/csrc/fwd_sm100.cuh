@@ -38,7 +38,7 @@ struct FwdKParams {
   int H, N;
   int n_qt, n_units;   // query tiles per (batch, head) unit, number of units: the grid has n_qt * n_units blocks
   int unit_group;      // units per group of the block order
-  int D;       // head dimension of the tensors (the kernel is compiled for it rounded up to 64 or 128)
+  int D;       // head dimension of the tensors (the kernel is compiled for it rounded up to 64, 128 or 256)
   int causal;
   float c1;      // sm_scale * log2(e)
   float s;       // sm_scale
